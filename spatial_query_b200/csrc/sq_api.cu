@@ -99,7 +99,7 @@ int32_t nearest_core(sq_ctx* ctx, const sq_bvh* b, bool cast, const float* d_q, 
     return near_first_launch(ctx, b, b->ks.ray_nearest_regtop, ref_fn, p, b->depth);
   if (!cast && !stats && ctx->layout == SQ_LAYOUT_BINARY_VOTE && b->ks.ray_nearest_vote)
     return near_first_launch(ctx, b, b->ks.ray_nearest_vote, ref_fn, p, b->depth);
-  return near_first_launch(ctx, b, near_fn, kReplayInKernel ? nullptr : ref_fn, p, b->depth);
+  return near_first_launch(ctx, b, near_fn, ref_fn, p, b->depth);
 }
 
 int32_t list_core(sq_ctx* ctx, const sq_bvh* b, int kind, const float* d_q, uint32_t n, float max_toi,
@@ -365,7 +365,7 @@ static int32_t upload_impl(sq_ctx* ctx, int32_t dim, int32_t narrow, uint32_t n_
   b->n_nodes = n_nodes;
   b->n_prims = n_prims;
   b->stride = prim_stride;
-  b->prim_vec = custom ? (prim_stride + 2 * dim + 1 + 3) / 4 : prim_vec(dim, narrow);
+  b->prim_vec = custom ? record_vec(prim_stride + 2 * dim + 1) : prim_vec(dim, narrow);
   b->ks = ks;
   if (n_nodes == 0) {
     *out = b.release();
@@ -1315,7 +1315,7 @@ int32_t sqi::seeded_nearest(sq_ctx* ctx, const sq_bvh* b, const float* d_rays, u
     // above the bucket) while the bucket is searched: no deeper than a plain
     // descent to the same node, so the tree's depth bounds the stack.
     if ((rc = near_first_launch(ctx, b, b->ks.ray_nearest_seeded[st ? 1 : 0],
-                                kReplayInKernel ? nullptr : b->ks.ray_nearest[1][st ? 1 : 0], p,
+                                b->ks.ray_nearest[1][st ? 1 : 0], p,
                                 b->depth + 1)))
       return rc;
   }
@@ -1433,14 +1433,6 @@ int32_t sqi::pipelined(sq_ctx* ctx, uint32_t n, const std::function<int32_t(uint
 int32_t sqi::near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, const void* ref_fn, QueryParams& p,
                                uint32_t stack) {
   p.window = ctx->window;
-  if (!ref_fn) {
-    // The kernel answers its uncertified queries again itself; only their
-    // number is kept.
-    CK(cudaMemsetAsync(ctx->d_replays, 0, sizeof(uint32_t), ctx->stream));
-    p.replay_count = ctx->d_replays;
-    p.replay_list = nullptr;
-    return launch_persistent(ctx, fn, p, stack, p.n);
-  }
   // The replay list holds at most every query of the batch; it grows here,
   // outside any stream capture once a batch of this size has run.
   const size_t need = size_t(std::max<uint32_t>(p.n, 1)) * sizeof(uint32_t);
@@ -1453,14 +1445,16 @@ int32_t sqi::near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, con
     ctx->replay_list.cap = need;
   }
   CK(cudaMemsetAsync(ctx->d_replays, 0, sizeof(uint32_t), ctx->stream));
+  const bool replays = b->narrow != SQ_NARROW_AABB;
+  uint32_t* counters = nullptr;
+  int32_t rc = work_counters(ctx, replays ? 2 : 1, &counters);
+  if (rc) return rc;
   p.replay_count = ctx->d_replays;
   p.replay_list = static_cast<uint32_t*>(ctx->replay_list.p);
-  p.window = ctx->window;
-  int32_t rc = launch_persistent(ctx, fn, p, stack, p.n);
-  if (rc) return rc;
+  if ((rc = launch_persistent(ctx, fn, p, stack, p.n, counters))) return rc;
   // A box leaf's hit is its own slab entry, so box answers are always
   // certified and nothing is ever appended: no replay launch.
-  if (b->narrow == SQ_NARROW_AABB) return SQ_OK;
+  if (!replays) return SQ_OK;
   // The uncertified queries again, in the reference order, unseeded.
   QueryParams r = p;
   r.replay_count = nullptr;
@@ -1468,7 +1462,7 @@ int32_t sqi::near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, con
   r.seed_bucket = nullptr;
   r.q_list = static_cast<const uint32_t*>(ctx->replay_list.p);
   r.q_count = ctx->d_replays;
-  return launch_persistent(ctx, ref_fn, r, b->depth, p.n);
+  return launch_persistent(ctx, ref_fn, r, b->depth, p.n, counters + 1);
 }
 
 // ============================================================================

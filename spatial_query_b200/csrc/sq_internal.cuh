@@ -103,9 +103,7 @@ namespace sqi {
 using namespace sq;
 
 // Near-first nearest launch `fn` followed by the reference-order replay
-// (`ref_fn`) of the queries it could not certify; with `ref_fn` null the
-// kernel answers those queries again itself (sq_api.cu).
-constexpr bool kReplayInKernel = SQ_REPLAY_IN_KERNEL && !SQ_POSTPONE_LEAVES;
+// (`ref_fn`) of the queries it could not certify (sq_api.cu).
 int32_t near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, const void* ref_fn, QueryParams& p,
                           uint32_t stack);
 
@@ -191,12 +189,12 @@ inline uint32_t stride_of(int dim, int narrow) {
 
 inline uint32_t prim_vec(int dim, int narrow) {
   uint32_t payload = narrow == SQ_NARROW_AABB ? 2 * dim : (narrow == SQ_NARROW_TRIANGLE ? 9 : dim + 1);
-  return (payload + 1 + 3) / 4;
+  return record_vec(payload + 1);
 }
 
-inline uint32_t node_vec(int dim) { return (4 * dim + 2 + 3) / 4; }
-inline uint32_t wide_vec(int dim) { return (8 * dim + 4 + 3) / 4; }
-inline uint32_t quant_vec(int dim) { return (dim + (dim + 3) / 4 + 2 * dim + 4 + 3) / 4; }
+inline uint32_t node_vec(int dim) { return record_vec(4 * dim + 2); }
+inline uint32_t wide_vec(int dim) { return record_vec(8 * dim + 4); }
+inline uint32_t quant_vec(int dim) { return record_vec(dim + (dim + 3) / 4 + 2 * dim + 4); }
 
 // Stream-ordered scratch on the context's stream from the context's own
 // memory pool. The pool keeps what is freed for the next call (no release
@@ -241,25 +239,39 @@ inline int occupancy(sq_ctx* ctx, const void* fn, size_t smem) {
   return nb;
 }
 
+// The next `count` work counters of the context's ring, zeroed on its stream
+// (one fill for a launch and the launch that follows it).
+inline int32_t work_counters(sq_ctx* ctx, uint32_t count, uint32_t** out) {
+  if (ctx->slot % kCounterSlots + count > kCounterSlots) ctx->slot = 0;
+  *out = ctx->d_counters + ctx->slot % kCounterSlots;
+  ctx->slot += count;
+  CK(cudaMemsetAsync(*out, 0, count * sizeof(uint32_t), ctx->stream));
+  return SQ_OK;
+}
+
 // The persistent grid: (resident blocks per SM) x (SM count), no more blocks
 // than the queries need. The traversal stack is dynamic shared memory sized
 // to the tree depth, so shallow trees leave room for more resident warps.
 // Launches a persistent kernel whose single parameter is *params (with its
-// counter and stack fields set here) on the context's stream.
+// counter and stack fields set here) on the context's stream. The work counter
+// is zeroed here unless the caller passes one that is.
 template <class Params>
-inline int32_t launch_persistent(sq_ctx* ctx, const void* fn, Params& p, uint32_t depth, uint64_t n);
-
-template <class Params>
-inline int32_t launch_persistent(sq_ctx* ctx, const void* fn, Params& p, uint32_t depth, uint64_t n) {
-  uint32_t* ctr = ctx->d_counters + (ctx->slot++ % kCounterSlots);
-  CK(cudaMemsetAsync(ctr, 0, sizeof(uint32_t), ctx->stream));
+inline int32_t launch_persistent(sq_ctx* ctx, const void* fn, Params& p, uint32_t depth, uint64_t n,
+                                 uint32_t* zeroed_counter = nullptr) {
+  uint32_t* ctr = zeroed_counter;
+  if (!ctr) {
+    int32_t rc = work_counters(ctx, 1, &ctr);
+    if (rc) return rc;
+  }
   p.counter = ctr;
   p.stack = int(std::max<uint32_t>(depth, 1));
   const size_t smem = size_t(p.stack) * kThreads * 8;
   if (smem > 48 * 1024) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   int bps = ctx->blocks_per_sm > 0 ? ctx->blocks_per_sm : occupancy(ctx, fn, smem);
-  uint64_t want = (n + kThreads - 1) / kThreads;
-  uint64_t grid = std::min<uint64_t>(uint64_t(ctx->sm_count) * bps, std::max<uint64_t>(want, 1));
+  // A warp takes at most its share of the queries (query_kernel's width): a
+  // batch smaller than the grid's lanes is spread over every resident warp.
+  const uint64_t most = uint64_t(ctx->sm_count) * bps;
+  const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>(most, (n + kThreads / 32 - 1) / (kThreads / 32)));
   void* args[] = {&p};
   CK(cudaLaunchKernel(fn, dim3(unsigned(grid)), dim3(kThreads), args, smem, ctx->stream));
   ctx->launches++;

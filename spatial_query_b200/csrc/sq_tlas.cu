@@ -268,7 +268,7 @@ extern "C" int32_t sq_blas_set_upload(sq_ctx* ctx, uint32_t n_blas, const uint32
   uint32_t node_off = 0;
   const uint32_t total_tris = n_blas ? tri_offsets[n_blas] : 0;
   if (total_tris >= kLeafBit) return fail(ctx, SQ_ERR_INVALID, "too many triangles");
-  prims.assign(size_t(total_tris) * 12, 0.f);
+  prims.assign(size_t(total_tris) * kBlasPrimVec * 4, 0.f);
   for (uint32_t b = 0; b < n_blas; ++b) {
     const uint32_t n0 = node_offsets[b], n1 = node_offsets[b + 1];
     const uint32_t t0 = tri_offsets[b], t1 = tri_offsets[b + 1];
@@ -304,7 +304,7 @@ extern "C" int32_t sq_blas_set_upload(sq_ctx* ctx, uint32_t n_blas, const uint32
       for (uint32_t j = 0; j < L.count; ++j) {
         const uint32_t pos = L.first + j;  // global
         const uint32_t id = prim_indices[pos];  // local to the mesh
-        float* r = prims.data() + size_t(pos) * 12;
+        float* r = prims.data() + size_t(pos) * kBlasPrimVec * 4;
         std::memcpy(r, tris + (size_t(t0) + id) * 9, 36);
         uint32_t w = id | (j + 1 == L.count ? kLeafBit : 0u);
         std::memcpy(&r[9], &w, 4);
@@ -407,7 +407,7 @@ extern "C" int32_t sq_tlas_upload(sq_ctx* ctx, int32_t dim, int32_t kind, uint32
 
   const int P = kind == SQ_INSTANCE_BOX ? D : 1;
   const int words = D * D + D + P + 2;
-  const int vec = (words + 3) / 4;
+  const int vec = record_vec(words);
   std::vector<float> insts(size_t(n_inst) * vec * 4, 0.f);
   std::vector<float> local(size_t(n_inst) * 2 * D), world(size_t(n_inst) * 2 * D);
   for (const RefitLeaf& L : C.leaves) {

@@ -43,8 +43,10 @@ template <int D, int IK> struct InstLayout {
   static constexpr int blas = D * D + D + P;
   static constexpr int id = D * D + D + P + 1;
   static constexpr int words = id + 1;
-  static constexpr int vec = (words + 3) / 4;
+  static constexpr int vec = record_vec(words);
 };
+
+constexpr int kBlasPrimVec = PrimLayout<3, kNarrowTri>::vec;  // BLAS triangle records
 
 struct BlasRoot {
   uint32_t code;
@@ -234,8 +236,8 @@ __device__ __forceinline__ bool blas_nearest(const TlasParams& p, uint32_t b, co
     if (done) break;
     uint32_t pos = code & ~kLeafBit;
     for (;;) {
-      float rec[12];
-      load_vec<3>(p.bprims + size_t(pos) * 3, rec);
+      float rec[kBlasPrimVec * 4];
+      load_vec<kBlasPrimVec>(p.bprims + size_t(pos) * kBlasPrimVec, rec);
       const uint32_t idw = __float_as_uint(rec[9]);
       const uint32_t id = idw & ~kLeafBit;
       float t, nrm[3];
@@ -679,8 +681,8 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
   auto blas_leaf = [&]() {
     uint32_t pos = L.code & ~kLeafBit;
     for (;;) {
-      float rec[12];
-      load_vec<3>(p.bprims + size_t(pos) * 3, rec);
+      float rec[kBlasPrimVec * 4];
+      load_vec<kBlasPrimVec>(p.bprims + size_t(pos) * kBlasPrimVec, rec);
       const uint32_t idw = __float_as_uint(rec[9]);
       const uint32_t id = idw & ~kLeafBit;
       float t, nrm[3];

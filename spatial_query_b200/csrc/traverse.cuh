@@ -77,16 +77,6 @@ constexpr int kThreads = 128;
 #ifndef SQ_REG_TOP
 #define SQ_REG_TOP 0
 #endif
-// Uncertified near-first answers answered again by the same lane at its
-// next refill (1), or listed for a reference-order launch (0, the default).
-// The lane replay removes the second launch (about 20 us per 1,048,576-ray
-// call, the serial walk of the one or two listed rays) but measured 0.918 ms
-// against 0.619 ms for the child-pair walk of the terrain's rays, with the
-// same single replay in both: the replay state in the refill loop costs the
-// whole walk far more than the launch it saves.
-#ifndef SQ_REPLAY_IN_KERNEL
-#define SQ_REPLAY_IN_KERNEL 0
-#endif
 // Child order by warp vote (1) in the certified near-first walk: the lanes
 // that open the same record with both children hit take the order most of
 // them prefer (a __match_any_sync group and a ballot), so lanes that agree
@@ -98,11 +88,23 @@ constexpr int kThreads = 128;
 #ifndef SQ_WARP_ORDER
 #define SQ_WARP_ORDER 0
 #endif
+// query_kernel's warp scheduling. Measured on the terrain (1,048,576
+// triangles and rays, each pair by the other values alike): answers written
+// and queries loaded once 1 / 4 / 8 / 16 / 24 lanes are free 705 / 641 / 625
+// / 615 / 617 us; a leaf pass once 1/2, 2/3, 1/3 or 1/4 of the walking lanes
+// wait at one 615 / 627 / 625 / 633 us.
+constexpr int kRefill = 16;     // free lanes (of 32) before the warp refills them
+constexpr int kLeafWeight = 2;  // a leaf pass when waiting lanes x this reach the walking lanes
 constexpr int kMaxStack = 96;  // deepest tree accepted (96 KB of stack per block)
+
+// 16-byte vectors of a record of `words` words: records longer than one
+// vector are padded to whole 32-byte sectors, so that each is read with
+// 32-byte loads (load_vec).
+__host__ __device__ constexpr int record_vec(int words) { return words <= 4 ? 1 : (words + 7) / 8 * 2; }
 
 template <int D> struct NodeLayout {
   static constexpr int words = 4 * D + 2;  // a.lo a.hi b.lo b.hi code_a code_b
-  static constexpr int vec = (words + 3) / 4;
+  static constexpr int vec = record_vec(words);
 };
 
 // Four-wide records (the binary tree with every other level folded into its
@@ -111,7 +113,7 @@ template <int D> struct NodeLayout {
 // subtrees the binary walk would, in half the dependent fetches.
 template <int D> struct WideLayout {
   static constexpr int words = 8 * D + 4;  // c0.lo c0.hi ... c3.lo c3.hi code0 .. code3
-  static constexpr int vec = (words + 3) / 4;
+  static constexpr int vec = record_vec(words);
 };
 
 // Quantised four-wide records: the same four-wide tree (same numbering and
@@ -129,7 +131,7 @@ template <int D> struct QuantLayout {
   static constexpr int o_q = D + exp_words;
   static constexpr int o_code = D + exp_words + 2 * D;
   static constexpr int words = o_code + 4;
-  static constexpr int vec = (words + 3) / 4;
+  static constexpr int vec = record_vec(words);
 };
 
 // origin + q x 2^e, in the arithmetic both the quantiser and the walk use.
@@ -222,7 +224,7 @@ template <int D, int N> struct PrimLayout {
                                  : (N == kNarrowCustom) ? SQ_CUSTOM_STRIDE + 2 * D
                                                         : D + 1;
   static constexpr int id_word = payload;
-  static constexpr int vec = (payload + 1 + 3) / 4;
+  static constexpr int vec = record_vec(payload + 1);
 };
 
 template <int K> struct QueryLayout {
@@ -298,14 +300,34 @@ __device__ __forceinline__ bool accepts(const QueryParams& p, uint32_t id) {
   return (__ldg(p.layers + id) & p.mask) != 0ull;
 }
 
+// A record of NV 16-byte vectors through the read-only path. Lanes of a warp
+// read records of their own, so every load instruction costs the L1 a lookup
+// per lane: 32-byte loads (sm_100) halve the lookups of 16-byte ones (terrain
+// 621 -> 601 us per 1,048,576 rays). Compilers before 12.9 do not know them;
+// the NVRTC that compiles a consumer's narrow phase can be older.
+#if __CUDACC_VER_MAJOR__ * 100 + __CUDACC_VER_MINOR__ >= 1209
+constexpr bool kWideLoads = true;
+#else
+constexpr bool kWideLoads = false;
+#endif
 template <int NV> __device__ __forceinline__ void load_vec(const float4* __restrict__ src, float* dst) {
+  if constexpr (kWideLoads && NV % 2 == 0) {
 #pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    float4 v = __ldg(src + j);
-    dst[4 * j + 0] = v.x;
-    dst[4 * j + 1] = v.y;
-    dst[4 * j + 2] = v.z;
-    dst[4 * j + 3] = v.w;
+    for (int j = 0; j < NV / 2; ++j) {
+      float* d = dst + 8 * j;
+      asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
+          : "l"(src + 2 * j));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      float4 v = __ldg(src + j);
+      dst[4 * j + 0] = v.x;
+      dst[4 * j + 1] = v.y;
+      dst[4 * j + 2] = v.z;
+      dst[4 * j + 3] = v.w;
+    }
   }
 }
 
@@ -318,8 +340,13 @@ template <int NV> __device__ __forceinline__ void load_vec(const float4* __restr
 // entry lies past the best hit by more than a small relative window (2^-16 by
 // default), which finds h whenever no hit is computed that far before the
 // entry of a box enclosing its primitive. A query whose answer comes before
-// its own primitive's AABB entry is not certified: it is appended to a list
-// that a second launch answers again in the reference order.
+// its own primitive's AABB entry e still has it if no other hit lies before e:
+// the reference's limit is then e or later until it reaches h (the query's
+// limit has to be, and e has to lie within the window, so that every hit
+// before it was seen). Otherwise the query is not certified: it is appended to
+// a list that a second launch answers again in the reference order, one lane
+// per query (1,048,576 rays against 100,000 balls: 489 queries without the
+// second rule, 87 with it).
 __device__ __forceinline__ float near_limit(float limit, float window) {
   return __fadd_rn(limit, __fadd_rn(__fmul_rn(fabsf(limit), window), 0x1p-20f));
 }
@@ -479,30 +506,56 @@ template <int D, int K> struct Lane {
   RayPre<D> r;
   float pmin[D], pmax[D];
   float limit;       // nodes whose entry lies past this are pruned (near-first: the best hit plus the window)
-  uint32_t best_pos; // near-first: primitive position of the best hit (for its certification)
+  uint32_t best_pos; // primitive position of the best hit (its certification and normal)
   uint32_t q;
   uint32_t code;
   float code_t;      // entry of the node in code (postponed-leaf walks re-check it after a leaf)
   uint32_t top_code; // postponed-leaf walks: the stack's top entry, held in registers
   float top_t;
   bool has_top;
-  bool ref;          // this walk answers the query again in the crate's own order (unseeded, exact limit)
   int sp;
   bool fast;
   uint32_t best_leaf;
   float best_t;
-  float best_n[D];
+  float second_t;    // near-first: the nearest of the query's other hits
+  float best_n[D];   // consumer narrow phases only
   uint32_t count;
   unsigned long long csr_base;
   uint32_t v_nodes, v_nar, v_hit;
 };
 
-// The persistent query kernel. Each warp keeps 32 queries in flight; a lane
-// whose query finishes takes the next one from the shared counter at the top
-// of the loop (one atomic per warp per refill), so a warp never idles on its
-// slowest query. Between refills a lane descends interior records until it
-// reaches a leaf, tests that leaf's primitives and pops the next waiting
-// child (Aila and Laine's while-while loop with dynamic fetch).
+// Resident blocks per SM that query_kernel's registers are held to: what the
+// walk itself needs (the code that runs once per query or once per launch may
+// spill). At D = 3 and 1,048,576 terrain rays, 7 / 8 / 9 / 10 blocks measured
+// 512 / 464 / 441 / 483 us (nine: 56 registers, no spills; ten: 48 registers,
+// 32 bytes spilled). Longer rays and records (D = 4 and 6, casts, four-wide
+// records) need more registers each.
+__host__ __device__ constexpr int resident_blocks(int D, int kind, bool stats, bool wide) {
+  if (stats) return 1;
+  if (wide) return D <= 3 ? 8 : (D == 4 ? 6 : 5);
+  if (D <= 3 || kind == kOverlap) return 9;
+  if (kind == kCastNearest || kind == kCastAll) return D == 4 ? 7 : 5;
+  return D == 4 ? 8 : 7;
+}
+
+// The persistent query kernel. Each warp keeps up to 32 queries in flight and
+// its lanes step together: a pass tests one record for every lane at an
+// interior node, or the primitives of one leaf for every lane at a leaf,
+// whichever more lanes wait for (a lane that reaches its leaf early waits for
+// company), and the lanes whose queries have ended are refilled together from
+// the shared counter (one atomic per refill). A lane visits what it would
+// visit alone, in the same order. On the terrain 16.3 of 32 threads are active
+// per warp instruction (7.5 when each lane descended to its own leaf before
+// the warp tested leaves); the kernel now issues 2.57 instructions per cycle
+// and SM, with the L1's data pipe 69% busy.
+//
+// A launch ends on its longest queries, dependent chains of hundreds of
+// fetches at some 0.3 us each. HELP walks split them over the lanes that have
+// no query left (see the tail of the kernel), and a batch smaller than the
+// grid's lanes is dealt out thinly over every warp, so that each query has
+// free lanes beside it from the start. Both together with the passes above:
+// terrain 632 -> 441 us per 1,048,576 rays, 100,003 filtered ball casts 268
+// -> 150 us, 256 rays against 10,000 boxes 135 -> 26 us.
 //
 // SEED (nearest rays only): the learned guide's predicted bucket, a subtree
 // at a fixed depth, is searched first; its nearest hit becomes the limit for
@@ -519,7 +572,7 @@ template <int D, int K> struct Lane {
 // order by warp vote.
 template <int D, int N, int K, bool REF, bool STATS, bool SEED = false, bool WIDE = false, bool QUANT = false,
           int WALK = 0>
-__global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
+__global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) query_kernel(const QueryParams p) {
   static_assert(!WIDE || (K == kRayNearest && !REF && !STATS && !SEED), "four-wide walks serve near-first rays only");
   static_assert(!QUANT || WIDE, "quantised records are a four-wide layout");
   constexpr bool kNearest = (K == kRayNearest || K == kCastNearest);
@@ -542,7 +595,6 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
 
   unsigned long long c_vis = 0, c_nar = 0, c_hit = 0;
   Lane<D, K> L;
-  bool live = false, exhausted = false;
   const uint32_t n_queries = p.q_count ? *p.q_count : p.n;
 
   constexpr bool DETECT = kNearest && !REF;
@@ -551,13 +603,9 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
   // walks keep the crate's sequence.
   constexpr bool SPEC = (SQ_POSTPONE_LEAVES || WALK == 1) && DETECT && !STATS && !WIDE;
   constexpr bool kRegTop = SQ_REG_TOP || WALK == 1;
-  // An uncertified answer is answered again by the same lane, in the crate's
-  // order over the child-pair records, at its next refill (no second launch
-  // walking a handful of rays while the GPU idles). Four-wide walks list
-  // such queries for a reference-order launch over the child-pair records.
-  constexpr bool INREPLAY = SQ_REPLAY_IN_KERNEL && DETECT && !WIDE && !SPEC;
-  bool pending = false;
-  uint32_t pending_q = 0;
+  // Idle lanes help where the answer does not depend on the order of the
+  // visits and no counter reports them.
+  constexpr bool HELP = DETECT && !STATS && !SPEC;
   const float kInf = __int_as_float(0x7f800000);
 
   // Box test of one child (or the root) against the lane's query: the slab
@@ -582,7 +630,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
 
   // Pops the next waiting child whose entry still lies within the limit
   // (exactly the reference's slab verdict at pop time). False: stack empty.
-  auto pop = [&]() -> bool {
+  auto pop = [&](int lo) -> bool {
     if constexpr (SPEC && kRegTop) {
       if (L.has_top) {
         L.has_top = false;
@@ -591,7 +639,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
         if (L.top_t <= L.limit) return true;
       }
     }
-    while (L.sp > 0) {
+    while (L.sp > lo) {
       --L.sp;
       L.code = s_code[L.sp * kThreads + tid];
       const float t = s_t[L.sp * kThreads + tid];
@@ -603,26 +651,28 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
 
   auto finish = [&]() {
     const uint32_t q = L.q;
-    if constexpr (DETECT && N != kNarrowAabb) {
-      // Certify the answer: not before its own primitive's AABB entry.
-      if (L.best_leaf != kNoHit && !L.ref) {
+    float nrm[D];
+    if constexpr (kNearest) {
+#pragma unroll
+      for (int i = 0; i < D; ++i) nrm[i] = N == kNarrowCustom ? L.best_n[i] : 0.f;
+      if (L.best_leaf != kNoHit && ((DETECT && N != kNarrowAabb) || (N != kNarrowCustom && p.out_normal))) {
         float rec[PL::vec * 4];
         load_vec<PL::vec>(p.prims + size_t(L.best_pos) * PL::vec, rec);
-        if (L.best_t < prim_entry<D, N, kCast>(rec, L.r, L.pmin, L.pmax, L.fast)) {
-          if constexpr (INREPLAY) {
-            // Answered again by this lane in the crate's order; this walk's
-            // counters still count, its answer is not written.
-            pending = true;
-            pending_q = q;
-            if (p.replay_count) atomicAdd(p.replay_count, 1u);
-            if (STATS) {
-              c_vis += L.v_nodes;
-              c_nar += L.v_nar;
-              c_hit += L.v_hit;
-            }
-            return;
-          } else {
+        // Certify the answer: not before its own primitive's AABB entry.
+        if constexpr (DETECT && N != kNarrowAabb) {
+          const float te = prim_entry<D, N, kCast>(rec, L.r, L.pmin, L.pmax, L.fast);
+          const float mt = p.max_toi_arr ? p.max_toi_arr[q] : p.max_toi;
+          if (L.best_t < te && !(te <= mt && te <= near_limit(L.best_t, p.window) && te <= L.second_t))
             p.replay_list[atomicAdd(p.replay_count, 1u)] = q;
+        }
+        // The best hit's normal, once per query: the same test of the same
+        // primitive bounded by the hit itself.
+        if constexpr (N != kNarrowCustom) {
+          if (p.out_normal) {
+            float t;
+            if constexpr (kCast) narrow_cast<D, N>(rec, L.r, L.pmin, L.pmax, L.best_t, t, nrm);
+            else if constexpr (N == kNarrowTri) tri_normal(rec, rec + 3, rec + 6, nrm);
+            else narrow_ray<D, N>(rec, L.r, L.best_t, t, nrm);
           }
         }
       }
@@ -633,7 +683,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
       if (p.out_sub) p.out_sub[q] = (L.best_leaf != kNoHit && p.sub) ? __ldg(p.sub + L.best_leaf) : kNoHit;
       if (p.out_normal) {
 #pragma unroll
-        for (int i = 0; i < D; ++i) p.out_normal[size_t(q) * D + i] = L.best_n[i];
+        for (int i = 0; i < D; ++i) p.out_normal[size_t(q) * D + i] = nrm[i];
       }
       if (p.out_point) {
         float pt[D];
@@ -674,9 +724,8 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
   };
 
   // Loads query q and tests the root. False when the query is already done.
-  auto start = [&](uint32_t q, bool ref) -> bool {
+  auto start = [&](uint32_t q) -> bool {
     L.q = q;
-    L.ref = ref;
     const float* src = p.queries + size_t(q) * QW;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
@@ -702,8 +751,11 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
     }
     L.best_leaf = kNoHit;
     L.best_t = 0.f;
+    L.second_t = kInf;
+    if constexpr (N == kNarrowCustom) {
 #pragma unroll
-    for (int i = 0; i < D; ++i) L.best_n[i] = 0.f;
+      for (int i = 0; i < D; ++i) L.best_n[i] = 0.f;
+    }
     L.count = 0;
     L.csr_base = 0;
     if constexpr (K == kOverlap) {
@@ -753,7 +805,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
     float te;
     const bool hit_root = test_box(lo, hi, te);
     L.code_t = te;
-    if constexpr (SEED) if (!L.ref) {
+    if constexpr (SEED) {
       const int32_t bk = p.seed_bucket[q];
       if (hit_root && bk >= 0 && uint32_t(bk) < p.n_buckets) {
         const uint2 e = __ldg(p.buckets + bk);
@@ -805,12 +857,26 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
     return hit_root;
   };
 
-  // Tests the primitives of the leaf in L.code.
-  auto leaf = [&](uint32_t code) {
-    uint32_t pos = code & ~kLeafBit;
-    for (;;) {
-      float rec[PL::vec * 4];
-      load_vec<PL::vec>(p.prims + size_t(pos) * PL::vec, rec);
+  // A hit of the lane's query: kept when it is before the best one.
+  auto take_hit = [&](float t, uint32_t id, uint32_t pos) -> bool {
+    const bool first = L.best_leaf == kNoHit || hit_before(t, id, L.best_t, L.best_leaf);
+    if constexpr (DETECT && N != kNarrowAabb) {
+      // The nearest of the other hits; a NaN marks the query uncertified.
+      const float other = first ? (L.best_leaf == kNoHit ? kInf : L.best_t) : t;
+      if (!(other >= L.second_t)) L.second_t = other == other ? other : -kInf;
+    }
+    if (first) {
+      L.best_leaf = id;
+      L.best_t = t;
+      L.best_pos = pos;
+      L.limit = DETECT ? near_limit(t, p.window) : t;
+    }
+    return first;
+  };
+
+  // Tests the primitive record at position pos. True: the last of its leaf.
+  auto prim = [&](const float* rec, uint32_t pos) -> bool {
+    {
       const uint32_t idw = __float_as_uint(rec[PL::id_word]);
       const uint32_t id = idw & ~kLeafBit;
       if (accepts(p, id)) {
@@ -841,17 +907,11 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
             else h = narrow_cast<D, N>(rec, L.r, L.pmin, L.pmax, L.limit, t, nrm);
             if (h) {
               if (STATS) L.v_hit += 1;
-              if (L.best_leaf == kNoHit || hit_before(t, id, L.best_t, L.best_leaf)) {
-                L.best_leaf = id;
-                L.best_t = t;
-                if (DETECT && !L.ref) {
-                  L.limit = near_limit(t, p.window);
-                  L.best_pos = pos;
-                } else {
-                  L.limit = t;
-                }
+              if (take_hit(t, id, pos)) {
+                if constexpr (N == kNarrowCustom) {  // a consumer's normal is the one its own test gave
 #pragma unroll
-                for (int i = 0; i < D; ++i) L.best_n[i] = nrm[i];
+                  for (int i = 0; i < D; ++i) L.best_n[i] = nrm[i];
+                }
               }
             }
           } else if constexpr (K == kRayAll) {
@@ -909,41 +969,200 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
           }
         }
       }
-      if (idw & kLeafBit) break;
-      ++pos;
+      return (idw & kLeafBit) != 0u;
+    }
+  };
+  // Tests the primitives of a leaf.
+  auto leaf = [&](uint32_t code) {
+    for (uint32_t pos = code & ~kLeafBit;; ++pos) {
+      float rec[PL::vec * 4];
+      load_vec<PL::vec>(p.prims + size_t(pos) * PL::vec, rec);
+      if (prim(rec, pos)) break;
     }
   };
 
-  for (;;) {
-    // Refill the lanes without a query.
-    const bool need = !live && !exhausted && !pending;
-    const uint32_t need_mask = __ballot_sync(FULL, need);
-    uint32_t qs = kNoHit;
-    if (need_mask) {
-      const int leader = __ffs(need_mask) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(p.counter, uint32_t(__popc(need_mask)));
-      base = __shfl_sync(FULL, base, leader);
-      if (need) {
-        const uint32_t q = base + uint32_t(__popc(need_mask & lt_mask));
-        if (q < n_queries) qs = p.q_list ? p.q_list[q] : q;
-        else exhausted = true;
+  // One record of the node in L.code: its overlapping children. True: the
+  // query has nothing left to visit (its stack is empty down to lo).
+  auto node_step = [&](int lo) -> bool {
+    if constexpr (WIDE) {
+      float t4[4];
+      uint32_t c4[4];
+      bool exact = true;
+      if constexpr (QUANT) {
+        if (scene_finite) {
+          // Decode each child's box (rounded outward) and test it.
+          using QL = QuantLayout<D>;
+          float qf[QL::vec * 4];
+          load_vec<QL::vec>(p.qnodes + size_t(L.code) * QL::vec, qf);
+          uint32_t qw[QL::vec * 4];
+#pragma unroll
+          for (int w = 0; w < QL::vec * 4; ++w) qw[w] = __float_as_uint(qf[w]);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            c4[k] = qw[QL::o_code + k];
+            float lo[D], hi[D];
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+              const float step = q_step(q_byte(qw + QL::o_exp, i));
+              lo[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + i), step);
+              hi[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + D + i), step);
+            }
+            float te = kInf;
+            if (c4[k] == kNoHit || !test_box(lo, hi, te)) {
+              c4[k] = kNoHit;
+              te = kInf;
+            }
+            t4[k] = te;
+          }
+          exact = false;
+        }
+      }
+      if (exact) {
+        float rec[WL::vec * 4];
+        load_vec<WL::vec>(p.wnodes + size_t(L.code) * WL::vec, rec);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          c4[i] = __float_as_uint(rec[8 * D + i]);
+          float te = kInf;
+          if (c4[i] == kNoHit || !test_box(rec + 2 * D * i, rec + 2 * D * i + D, te)) {
+            c4[i] = kNoHit;
+            te = kInf;
+          }
+          t4[i] = te;
+        }
+      }
+      // Ascending entry order (a five-comparator network); misses sort last.
+      auto cswap = [&](int a, int b) {
+        if (t4[b] < t4[a]) {
+          const float t = t4[a];
+          t4[a] = t4[b];
+          t4[b] = t;
+          const uint32_t c = c4[a];
+          c4[a] = c4[b];
+          c4[b] = c;
+        }
+      };
+      cswap(0, 1);
+      cswap(2, 3);
+      cswap(0, 2);
+      cswap(1, 3);
+      cswap(1, 2);
+#pragma unroll
+      for (int i = 3; i >= 1; --i) {
+        if (c4[i] != kNoHit) {
+          s_code[L.sp * kThreads + tid] = c4[i];
+          s_t[L.sp * kThreads + tid] = t4[i];
+          ++L.sp;
+        }
+      }
+      if (c4[0] != kNoHit) {
+        L.code = c4[0];
+      } else {
+        return !pop(lo);
+      }
+      return false;
+    }
+    float rec[NL::vec * 4];
+    load_vec<NL::vec>(p.nodes + size_t(L.code) * NL::vec, rec);
+    const uint32_t ca = __float_as_uint(rec[4 * D]);
+    const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
+    float ta, tb;
+    const bool pa = test_box(rec, rec + D, ta);
+    const bool pb = test_box(rec + 2 * D, rec + 3 * D, tb);
+    if (STATS) L.v_nodes += 2;
+    if constexpr (K == kOverlap) {
+      // A region heavier than the budget goes to the block-per-region
+      // kernel instead of holding the launch's tail on one thread.
+      if (p.heavy_list && !p.fill && ++L.v_nar > p.visit_budget) {
+        p.heavy_flag[L.q] = 1;
+        p.heavy_list[atomicAdd(p.heavy_count, 1u)] = L.q;
+        return true;
       }
     }
-    bool replay = false;
-    if (INREPLAY && pending) {
-      qs = pending_q;
-      pending = false;
-      replay = true;
+    if (pa && pb) {
+      // Reference order: child_a waits, child_b goes first. Near-first:
+      // the smaller entry goes first.
+      bool a_first = (REF || !kNearest || (SEED && p.far_first)) ? false : (ta <= tb);
+      if constexpr ((SQ_WARP_ORDER || WALK == 2) && DETECT && !WIDE) {
+        const bool voter = !(SEED && p.far_first);
+        const uint32_t voters = __ballot_sync(__activemask(), voter);
+        if (voter) {
+          const uint32_t same = __match_any_sync(voters, L.code);
+          const uint32_t yes = __ballot_sync(voters, a_first) & same;
+          a_first = 2 * __popc(yes) >= __popc(same);
+        }
+      }
+      s_code[L.sp * kThreads + tid] = a_first ? cb : ca;
+      s_t[L.sp * kThreads + tid] = a_first ? tb : ta;
+      ++L.sp;
+      L.code = a_first ? ca : cb;
+    } else if (pa) {
+      L.code = ca;
+    } else if (pb) {
+      L.code = cb;
+    } else {
+      return !pop(lo);
     }
-    if (qs != kNoHit) {
-      live = start(qs, replay);
-      if (!live) finish();
+    return false;
+  };
+
+  // The warp steps together: each pass either tests one record for every lane
+  // at an interior node or one leaf for every lane at a leaf, whichever more
+  // lanes wait for, so a lane that reaches its leaf early waits for company
+  // instead of running its primitives in a nearly empty warp. A lane whose
+  // query ends keeps its answer until kRefill lanes are free; then the answers
+  // are written and the next queries loaded together.
+  const uint32_t warps = gridDim.x * (kThreads / 32);
+  const int width = int(min(32u, max(1u, (n_queries + warps - 1) / warps)));
+  const uint32_t width_mask = width >= 32 ? FULL : (1u << width) - 1u;
+  const int refill = max(1, width * kRefill / 32);
+  bool live = false;       // the lane walks a query
+  bool held = false;       // the lane's query has ended, its answer is not written yet
+  bool exhausted = false;  // no query is left to take (the same for the whole warp)
+  // One pass over the walking lanes; a lane whose query has nothing left above
+  // stack entry lo stops walking.
+  auto step = [&](uint32_t live_mask, int lo) {
+    const bool at_leaf = live && (L.code & kLeafBit);
+    bool more = true;
+    const uint32_t leaf_mask = __ballot_sync(FULL, at_leaf);
+    if (__popc(leaf_mask) * kLeafWeight >= __popc(live_mask)) {
+      if (at_leaf) {
+        leaf(L.code);
+        more = pop(lo);
+      }
+    } else if (live && !at_leaf) {
+      more = !node_step(lo);
     }
-    const uint32_t live_mask = __ballot_sync(FULL, live);
-    if (!live_mask) {
-      if (__all_sync(FULL, exhausted)) break;
-      continue;
+    if (!more) {
+      live = false;
+      held = true;
+    }
+  };
+  for (;;) {
+    uint32_t live_mask = __ballot_sync(FULL, live);
+    const uint32_t idle_mask = width_mask & ~live_mask;
+    const int idle = __popc(idle_mask);
+    if (live_mask == 0u || (!exhausted && idle >= refill)) {
+      if (held) {
+        finish();
+        held = false;
+      }
+      if (exhausted) break;  // no lane walks and none holds an answer
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(p.counter, uint32_t(idle));
+      base = __shfl_sync(FULL, base, 0);
+      if ((idle_mask >> lane) & 1u) {
+        const uint32_t q = base + uint32_t(__popc(idle_mask & lt_mask));
+        if (q < n_queries) {
+          live = start(p.q_list ? p.q_list[q] : q);
+          held = !live;
+        }
+      }
+      // A batch smaller than the grid's lanes is dealt out in one round.
+      exhausted = width < 32 || base + uint32_t(idle) >= n_queries;
+      if (HELP && exhausted) break;
+      live_mask = __ballot_sync(FULL, live);
+      if (live_mask == 0u) continue;
     }
     if constexpr (SPEC) {
       if (live) {
@@ -961,7 +1180,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
             if (L.code & kLeafBit) {
               if (pend == kNoHit) {
                 pend = L.code;
-                if (!pop()) empty = true;
+                if (!pop(0)) empty = true;
               }
             } else {
               float rec[NL::vec * 4];
@@ -997,7 +1216,7 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
               } else if (pb) {
                 L.code = cb;
                 L.code_t = tb;
-              } else if (!pop()) {
+              } else if (!pop(0)) {
                 empty = true;
               }
             }
@@ -1007,147 +1226,117 @@ __global__ void __launch_bounds__(kThreads) query_kernel(const QueryParams p) {
         if (pend != kNoHit) leaf(pend);
         // The node after the leaf was taken with the limit as it stood:
         // drop it (and what follows, as pop does) if the leaf's hit prunes it.
-        if (!empty && L.code_t > L.limit && !pop()) empty = true;
+        if (!empty && L.code_t > L.limit && !pop(0)) empty = true;
         if (empty) {
           live = false;
+          held = true;
+        }
+      }
+    } else {
+      step(live_mask, 0);
+    }
+  }
+
+  if constexpr (HELP) {
+    // No query is left to take: the lanes without one now help the others of
+    // their warp. Every second pass while few lanes walk, else every fourth
+    // (256 rays against 10,000 boxes: 25.6 us at 2, 30.5 at 4; 100,003 casts:
+    // 157 and 149), a free lane copies a walking lane's query and takes over
+    // the bottom entry of its stack (the largest waiting subtree); what it
+    // finds goes back to the query's own lane, whose limit its helpers follow.
+    // The subtrees are disjoint and near-first answers are certified whatever
+    // the order of the visits, so the answers are the same.
+    __shared__ uint8_t s_donor[kThreads];
+    int owner = lane;  // the lane whose query this one walks
+    int lo = 0;        // stack entries below this one have been taken over
+    for (uint32_t pass = 0;; ++pass) {
+      uint32_t live_mask = __ballot_sync(FULL, live);
+      if (live_mask == 0u || ((pass & (__popc(live_mask) <= 8 ? 1u : 3u)) == 0u && live_mask != FULL)) {
+        // Hits of the helpers go to their owners, one at a time (they are few).
+        uint32_t found = __ballot_sync(FULL, owner != lane && L.best_leaf != kNoHit);
+        while (found) {
+          const int h = __ffs(found) - 1;
+          found &= found - 1u;
+          const int to = __shfl_sync(FULL, owner, h);
+          const float t = __shfl_sync(FULL, L.best_t, h);
+          const float t2 = __shfl_sync(FULL, L.second_t, h);
+          const uint32_t id = __shfl_sync(FULL, L.best_leaf, h);
+          const uint32_t pos = __shfl_sync(FULL, L.best_pos, h);
+          float n[D];
+          if constexpr (N == kNarrowCustom) {
+#pragma unroll
+            for (int i = 0; i < D; ++i) n[i] = __shfl_sync(FULL, L.best_n[i], h);
+          }
+          if (lane == to) {
+            if (take_hit(t, id, pos)) {
+              if constexpr (N == kNarrowCustom) {
+#pragma unroll
+                for (int i = 0; i < D; ++i) L.best_n[i] = n[i];
+              }
+            }
+            if (t2 < L.second_t) L.second_t = t2;
+          } else if (lane == h) {
+            L.best_leaf = kNoHit;
+            L.second_t = kInf;
+          }
+        }
+        L.limit = fminf(L.limit, __shfl_sync(FULL, L.limit, owner));
+        // A query that no lane walks any more is answered.
+        if (!live && owner != lane) owner = lane;  // a helper that has finished is free
+        uint32_t walked = 0u;                       // owners of the walking lanes
+        if (live) walked = 1u << owner;
+        walked = __reduce_or_sync(FULL, walked);
+        if (held && !((walked >> lane) & 1u)) {
           finish();
+          held = false;
+        }
+        if (live_mask == 0u) break;
+        const bool free = !live && !held;
+        const uint32_t free_mask = __ballot_sync(FULL, free);
+        const uint32_t donors = __ballot_sync(FULL, live && L.sp > lo);
+        if (free_mask != 0u && donors != 0u) {
+          const int nd = __popc(donors), nf = __popc(free_mask);
+          const int rank = __popc((((donors >> lane) & 1u) ? donors : free_mask) & lt_mask);
+          if ((donors >> lane) & 1u) s_donor[(tid & ~31) + rank] = uint8_t(lane);
+          __syncwarp();
+          const int e = rank / nd;
+          const int from = free ? s_donor[(tid & ~31) + rank % nd] : lane;
+          const int d_lo = __shfl_sync(FULL, lo, from);
+          const int d_sp = __shfl_sync(FULL, L.sp, from);
+          const bool taken = free && d_lo + e < d_sp;
+#pragma unroll
+          for (int i = 0; i < D; ++i) {
+            L.r.o[i] = __shfl_sync(FULL, L.r.o[i], from);
+            L.r.d[i] = __shfl_sync(FULL, L.r.d[i], from);
+            L.r.inv[i] = __shfl_sync(FULL, L.r.inv[i], from);
+            if constexpr (kCast) {
+              L.pmin[i] = __shfl_sync(FULL, L.pmin[i], from);
+              L.pmax[i] = __shfl_sync(FULL, L.pmax[i], from);
+            }
+          }
+          L.r.par = __shfl_sync(FULL, L.r.par, from);
+          L.fast = __shfl_sync(FULL, int(L.fast), from) != 0;
+          L.limit = __shfl_sync(FULL, L.limit, from);
+          const int d_owner = __shfl_sync(FULL, owner, from);
+          if (taken) {
+            const int at = (d_lo + e) * kThreads + (tid & ~31) + from;
+            L.code = s_code[at];
+            L.code_t = s_t[at];
+            L.best_leaf = kNoHit;
+            L.second_t = kInf;
+            L.sp = 0;
+            lo = 0;
+            owner = d_owner;
+            live = L.code_t <= L.limit;
+            if (!live) owner = lane;
+          }
+          __syncwarp();
+          if ((donors >> lane) & 1u) lo += min(L.sp - lo, (nf - rank + nd - 1) / nd);
+          live_mask = __ballot_sync(FULL, live);
         }
       }
-    } else if (live) {
-      bool done = false;
-      // Descend interior records until a leaf comes up.
-      while (!(L.code & kLeafBit)) {
-        if constexpr (WIDE) {
-          float t4[4];
-          uint32_t c4[4];
-          bool exact = true;
-          if constexpr (QUANT) {
-            if (scene_finite) {
-              // Decode each child's box (rounded outward) and test it.
-              using QL = QuantLayout<D>;
-              float qf[QL::vec * 4];
-              load_vec<QL::vec>(p.qnodes + size_t(L.code) * QL::vec, qf);
-              uint32_t qw[QL::vec * 4];
-#pragma unroll
-              for (int w = 0; w < QL::vec * 4; ++w) qw[w] = __float_as_uint(qf[w]);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                c4[k] = qw[QL::o_code + k];
-                float lo[D], hi[D];
-#pragma unroll
-                for (int i = 0; i < D; ++i) {
-                  const float step = q_step(q_byte(qw + QL::o_exp, i));
-                  lo[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + i), step);
-                  hi[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + D + i), step);
-                }
-                float te = kInf;
-                if (c4[k] == kNoHit || !test_box(lo, hi, te)) {
-                  c4[k] = kNoHit;
-                  te = kInf;
-                }
-                t4[k] = te;
-              }
-              exact = false;
-            }
-          }
-          if (exact) {
-            float rec[WL::vec * 4];
-            load_vec<WL::vec>(p.wnodes + size_t(L.code) * WL::vec, rec);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              c4[i] = __float_as_uint(rec[8 * D + i]);
-              float te = kInf;
-              if (c4[i] == kNoHit || !test_box(rec + 2 * D * i, rec + 2 * D * i + D, te)) {
-                c4[i] = kNoHit;
-                te = kInf;
-              }
-              t4[i] = te;
-            }
-          }
-          // Ascending entry order (a five-comparator network); misses sort last.
-          auto cswap = [&](int a, int b) {
-            if (t4[b] < t4[a]) {
-              const float t = t4[a];
-              t4[a] = t4[b];
-              t4[b] = t;
-              const uint32_t c = c4[a];
-              c4[a] = c4[b];
-              c4[b] = c;
-            }
-          };
-          cswap(0, 1);
-          cswap(2, 3);
-          cswap(0, 2);
-          cswap(1, 3);
-          cswap(1, 2);
-#pragma unroll
-          for (int i = 3; i >= 1; --i) {
-            if (c4[i] != kNoHit) {
-              s_code[L.sp * kThreads + tid] = c4[i];
-              s_t[L.sp * kThreads + tid] = t4[i];
-              ++L.sp;
-            }
-          }
-          if (c4[0] != kNoHit) {
-            L.code = c4[0];
-          } else if (!pop()) {
-            done = true;
-            break;
-          }
-          continue;
-        }
-        float rec[NL::vec * 4];
-        load_vec<NL::vec>(p.nodes + size_t(L.code) * NL::vec, rec);
-        const uint32_t ca = __float_as_uint(rec[4 * D]);
-        const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
-        float ta, tb;
-        const bool pa = test_box(rec, rec + D, ta);
-        const bool pb = test_box(rec + 2 * D, rec + 3 * D, tb);
-        if (STATS) L.v_nodes += 2;
-        if constexpr (K == kOverlap) {
-          // A region heavier than the budget goes to the block-per-region
-          // kernel instead of holding the launch's tail on one thread.
-          if (p.heavy_list && !p.fill && ++L.v_nar > p.visit_budget) {
-            p.heavy_flag[L.q] = 1;
-            p.heavy_list[atomicAdd(p.heavy_count, 1u)] = L.q;
-            done = true;
-            break;
-          }
-        }
-        if (pa && pb) {
-          // Reference order: child_a waits, child_b goes first. Near-first:
-          // the smaller entry goes first.
-          bool a_first = (REF || !kNearest || L.ref || (SEED && p.far_first)) ? false : (ta <= tb);
-          if constexpr ((SQ_WARP_ORDER || WALK == 2) && DETECT && !WIDE) {
-            const bool voter = !L.ref && !(SEED && p.far_first);
-            const uint32_t voters = __ballot_sync(__activemask(), voter);
-            if (voter) {
-              const uint32_t same = __match_any_sync(voters, L.code);
-              const uint32_t yes = __ballot_sync(voters, a_first) & same;
-              a_first = 2 * __popc(yes) >= __popc(same);
-            }
-          }
-          s_code[L.sp * kThreads + tid] = a_first ? cb : ca;
-          s_t[L.sp * kThreads + tid] = a_first ? tb : ta;
-          ++L.sp;
-          L.code = a_first ? ca : cb;
-        } else if (pa) {
-          L.code = ca;
-        } else if (pb) {
-          L.code = cb;
-        } else if (!pop()) {
-          done = true;
-          break;
-        }
-      }
-      if (!done) {
-        leaf(L.code);
-        done = !pop();
-      }
-      if (done) {
-        live = false;
-        finish();
-      }
+      step(live_mask, lo);
+      if (owner != lane) held = false;  // a helper has no answer of its own
     }
   }
   if (STATS) {
