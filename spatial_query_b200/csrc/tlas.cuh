@@ -46,7 +46,10 @@ template <int D, int IK> struct InstLayout {
   static constexpr int vec = record_vec(words);
 };
 
-constexpr int kBlasPrimVec = PrimLayout<3, kNarrowTri>::vec;  // BLAS triangle records
+// BLAS triangle records: 48 bytes, so that the records of a two-level scene
+// take less of the L2 (padded to 64: 3,081 against 3,067 us per frame of
+// 1,680,000 triangles).
+constexpr int kBlasPrimVec = 3;
 
 struct BlasRoot {
   uint32_t code;
@@ -179,111 +182,6 @@ __device__ __forceinline__ bool ray_local_box(const float* o, const float* d, co
   return true;
 }
 
-// A whole nearest query in BLAS b (Bvh::raycast_nearest, accel/bvh.rs:73-124)
-// for a local ray, on stack entries [base, ...).
-template <bool REF>
-__device__ __forceinline__ bool blas_nearest(const TlasParams& p, uint32_t b, const RayPre<3>& r, bool fast,
-                                             float mt, uint32_t* s_code, float* s_t, int tid, int base,
-                                             float& t_out, uint32_t& leaf_out, float* n_out, uint32_t& flag,
-                                             bool ref) {
-  const BlasRoot R = p.broots[b];
-  float limit = mt;
-  float cut = mt;  // near-first prunes past a small window beyond the limit (traverse.cuh)
-  const float kInf = __int_as_float(0x7f800000);
-  // The slab without the limit, then the entry against the cut.
-  auto test = [&](const float* lo, const float* hi, float& te) -> bool {
-    int ax;
-    const bool geo = fast ? slab_fast<3>(r, lo, hi, kInf, te) : slab<3>(r, lo, hi, kInf, te, ax);
-    return geo && te <= cut;
-  };
-  float te0;
-  if (!test(R.lo, R.hi, te0)) return false;
-  uint32_t code = R.code;
-  int sp = base;
-  uint32_t best = kNoHit;
-  float best_t = 0.f, best_n[3] = {0.f, 0.f, 0.f};
-  for (;;) {
-    bool done = false;
-    while (!(code & kLeafBit)) {
-      float rec[NodeLayout<3>::vec * 4];
-      load_vec<NodeLayout<3>::vec>(p.bnodes + size_t(code) * NodeLayout<3>::vec, rec);
-      const uint32_t ca = __float_as_uint(rec[12]);
-      const uint32_t cb = __float_as_uint(rec[13]);
-      float ta, tb;
-      const bool pa = test(rec, rec + 3, ta);
-      const bool pb = test(rec + 6, rec + 9, tb);
-      if (pa && pb) {
-        const bool a_first = REF ? false : (!ref && ta <= tb);
-        s_code[sp * kThreads + tid] = a_first ? cb : ca;
-        s_t[sp * kThreads + tid] = a_first ? tb : ta;
-        ++sp;
-        code = a_first ? ca : cb;
-      } else if (pa) {
-        code = ca;
-      } else if (pb) {
-        code = cb;
-      } else {
-        bool found = false;
-        while (sp > base) {
-          --sp;
-          code = s_code[sp * kThreads + tid];
-          const float t = s_t[sp * kThreads + tid];
-          if (t <= cut) { found = true; break; }
-        }
-        if (!found) { done = true; break; }
-      }
-    }
-    if (done) break;
-    uint32_t pos = code & ~kLeafBit;
-    for (;;) {
-      float rec[kBlasPrimVec * 4];
-      load_vec<kBlasPrimVec>(p.bprims + size_t(pos) * kBlasPrimVec, rec);
-      const uint32_t idw = __float_as_uint(rec[9]);
-      const uint32_t id = idw & ~kLeafBit;
-      float t, nrm[3];
-      if (ray_triangle(r.o, r.d, rec, rec + 3, rec + 6, t) && !(t > limit)) {
-        if (best == kNoHit || hit_before(t, id, best_t, best)) {
-          tri_normal(rec, rec + 3, rec + 6, nrm);
-          best = id;
-          best_t = t;
-          limit = t;
-          cut = t;
-          if (!REF && !ref) {
-            // certify the new best: not before its own triangle's AABB entry
-            float lo[3], hi[3], te;
-            int ax;
-            tri_aabb(rec, rec + 3, rec + 6, lo, hi);
-            if (fast) slab_fast<3>(r, lo, hi, kInf, te);
-            else slab<3>(r, lo, hi, kInf, te, ax);
-            flag = uint32_t(t < te);
-            cut = near_limit(t, p.window);
-          }
-          best_n[0] = nrm[0];
-          best_n[1] = nrm[1];
-          best_n[2] = nrm[2];
-        }
-      }
-      if (idw & kLeafBit) break;
-      ++pos;
-    }
-    bool found = false;
-    while (sp > base) {
-      --sp;
-      code = s_code[sp * kThreads + tid];
-      const float t = s_t[sp * kThreads + tid];
-      if (t <= cut) { found = true; break; }
-    }
-    if (!found) break;
-  }
-  if (best == kNoHit) return false;
-  t_out = best_t;
-  leaf_out = best;
-  n_out[0] = best_n[0];
-  n_out[1] = best_n[1];
-  n_out[2] = best_n[2];
-  return true;
-}
-
 template <int D> struct TLane {
   RayPre<D> r;  // world ray or cast path; regions keep lo in o and hi in d
   float pmin[D], pmax[D];
@@ -298,17 +196,21 @@ template <int D> struct TLane {
   bool fast;
   uint32_t best_leaf, best_sub;
   float best_t;
-  float best_n[D];
+  float best_n[D];    // box and ball instances
+  uint32_t best_pos;  // mesh instances: the best hit's instance and triangle
+  uint32_t best_tri;  // positions, from which its normal is made once
   uint32_t count;
   unsigned long long csr_base;
   uint32_t v_nodes, v_nar, v_hit;
 };
 
-// The mesh-instance walk (the two-level benchmark's kernel) is latency-bound
-// with divergent lanes, so resident warps count more than registers: it is
-// held to five resident blocks per SM (96 registers, a few spilled), which
-// measured 3.87 ms per two-level frame against 4.29 ms at six blocks (80
-// registers) and 3.89 ms at four.
+// The mesh-instance walk (the two-level benchmark's kernel) is bound by issue
+// and latency together (2.16 instructions per cycle and SM, 10.4 of 32 threads
+// active): five resident blocks per SM. Measured at 4 / 5 / 6 / 7 blocks: 3,766
+// / 3,067 / 3,039 / 3,550 us per frame of 1,000,000 rays, 262,144 casts and
+// 262,144 regions at 4,096 instances, 323 / 289 / 301 / 308 us per frame of
+// 20,000 of each at 500. Before the warp stepped together the frame took 4,086
+// us (6.4 threads active, 270 bytes of registers spilled at five blocks).
 template <int D, int IK, bool REF, bool STATS>
 __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) ? 5 : 1)
     tlas_kernel(const TlasParams p) {
@@ -329,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
 
   unsigned long long c_vis = 0, c_nar = 0, c_hit = 0;
   TLane<D> L;
-  bool live = false, exhausted = false;
+  L.code = 0u;
 
   auto is_ray = [&]() { return L.kind <= kTRayCross; };
   auto is_cast = [&]() { return L.kind == kTCastNearest || L.kind == kTCastAll; };
@@ -408,8 +310,10 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
     L.best_leaf = kNoHit;
     L.best_sub = kNoHit;
     L.best_t = 0.f;
+    if constexpr (IK != kInstMesh) {
 #pragma unroll
-    for (int i = 0; i < D; ++i) L.best_n[i] = 0.f;
+      for (int i = 0; i < D; ++i) L.best_n[i] = 0.f;
+    }
     L.count = 0;
     L.csr_base = (L.kind == kTOverlapFill) ? p.o_offsets[L.q] : 0ull;
     L.v_nodes = STATS ? 1u : 0u;
@@ -440,9 +344,30 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
       o_leaf[q] = L.best_leaf;
       if (o_toi) o_toi[q] = L.best_t;
       if (o_sub) o_sub[q] = L.best_sub;
-      if (o_nrm)
+      if (o_nrm) {
+        float n[D];
 #pragma unroll
-        for (int i = 0; i < D; ++i) o_nrm[size_t(q) * D + i] = L.best_n[i];
+        for (int i = 0; i < D; ++i) n[i] = IK == kInstMesh ? 0.f : L.best_n[i];
+        if constexpr (IK == kInstMesh) {
+          if (L.best_leaf != kNoHit) {
+            if (ray) {
+              float tri[kBlasPrimVec * 4], inst[IL::vec * 4], nl[3];
+              load_vec<kBlasPrimVec>(p.bprims + size_t(L.best_tri) * kBlasPrimVec, tri);
+              load_vec<IL::vec>(p.insts + size_t(L.best_pos) * IL::vec, inst);
+              tri_normal(tri, tri + 3, tri + 6, nl);
+              rotate<3>(inst + IL::rot, nl, n);
+            } else {
+              const float* w = p.world_aabbs + size_t(L.best_pos) * 2 * D;
+              float t;
+              int axis;
+              slab_grown<D>(L.r, w, w + D, L.pmin, L.pmax, L.best_t, t, axis);
+              entry_normal<D>(L.r.d, axis, n);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < D; ++i) o_nrm[size_t(q) * D + i] = n[i];
+      }
       if (o_pt) {
         float pt[D];
         if (L.best_leaf != kNoHit) {
@@ -484,7 +409,9 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
     return te;
   };
 
-  // `inner` is set when the instance's own nearest hit is not certified.
+  uint32_t b_tri = 0;  // position of the triangle hit in the BLAS being walked
+  // `inner` is set when the instance's own nearest hit is not certified. A mesh
+  // instance's normal is not kept: finish() makes it from b_tri.
   auto take = [&](float t, uint32_t id, uint32_t subv, const float* n, uint32_t pos, uint32_t inner) {
     if (is_nearest()) {
       if (L.best_leaf == kNoHit || hit_before(t, id, L.best_t, L.best_leaf)) {
@@ -497,8 +424,13 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
           L.flag = inner | uint32_t(t < inst_entry(pos));
           L.cut = near_limit(t, p.window);
         }
+        if constexpr (IK == kInstMesh) {
+          L.best_pos = pos;
+          L.best_tri = b_tri;
+        } else {
 #pragma unroll
-        for (int i = 0; i < D; ++i) L.best_n[i] = n[i];
+          for (int i = 0; i < D; ++i) L.best_n[i] = n[i];
+        }
       }
     } else if (L.kind == kTCastAll) {
       list_put<D>(p.c_k, p.c_leaf, p.c_toi, p.c_sub, p.c_normal, L.q, L.count, t, id, subv, n);
@@ -567,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
             hit = ray_ball<D, true>(L.r.o, L.r.d, tr, fadd(rec[IL::param], L.pmax[0]), L.limit, t, n);
           }
           if (hit) take(t, id, IK == kInstMesh ? kNoHit : subv, n, pos, 0u);
-        } else {
+        } else if constexpr (IK != kInstMesh) {  // rays at mesh instances walk their BLASes (unified below)
           if (STATS) L.v_nar += 1;
           // World ray -> instance space (tlas.rs:465-471).
           float v[D], lo[D], ld[D];
@@ -575,37 +507,7 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
           for (int i = 0; i < D; ++i) v[i] = fsub(L.r.o[i], tr[i]);
           rotate_t<D>(R, v, lo);
           rotate_t<D>(R, L.r.d, ld);
-          if constexpr (IK == kInstMesh) {
-            const float s = rec[IL::param];
-            RayPre<3> lr;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              lr.o[i] = fdiv(lo[i], s);
-              lr.d[i] = ld[i];
-            }
-            ray_prep<3>(lr);
-            bool f = p.blas_finite && lr.par == 0u && isfinite(s);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) f = f && isfinite(lr.o[i]) && isfinite(lr.d[i]);
-            float ts, nl[3];
-            uint32_t face;
-            const float mts = fdiv(L.limit, s);
-            uint32_t bflag = 0u;
-            // Only nearest queries are answered again when an instance's hit
-            // is not certified, so the others walk the BLAS in the crate's
-            // own order, whose answer needs no certificate.
-            const bool bh = blas_nearest<REF>(p, __float_as_uint(rec[IL::blas]), lr, f && !isnan(mts), mts, s_code,
-                                              s_t, tid, L.sp, ts, face, nl, bflag, L.ref || !is_nearest());
-            if (bh) {
-              const float toi = fmul(ts, s);
-              if (!(toi > L.limit)) {
-                float nw[3];
-                rotate<3>(R, nl, nw);
-                if (STATS) L.v_hit += 1;
-                take(toi, id, face, nw, pos, bflag);
-              }
-            }
-          } else if constexpr (IK == kInstBox) {
+          if constexpr (IK == kInstBox) {
             float t, nl[D], nw[D];
             if (ray_local_box<D>(lo, ld, rec + IL::param, L.limit, t, nl)) {
               rotate<D>(R, nl, nw);
@@ -655,12 +557,11 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
   // Mesh instances, rays (nearest, all hits, crossings): a lane walks its
   // instances' BLASes inside the same descent loop as the top level, one
   // leaf per pass, so that lanes in different levels and instances share
-  // the node-test instructions instead of each lane finishing a whole BLAS
-  // walk (blas_nearest) while the rest of its warp waits. Same visits, same
-  // order, same answers: nearest rays walk a BLAS near-first with the
-  // certificate, list rays walk it in the crate's own order (their
-  // instance hits are never answered again, so they need none) and list the
-  // instance's hit.
+  // the node-test instructions. Each BLAS walk is a whole nearest query
+  // (Bvh::raycast_nearest, accel/bvh.rs:73-124) on the stack entries above
+  // b_base: nearest rays walk it near-first with the certificate, list rays
+  // in the crate's own order (their instance hits are never answered again,
+  // so they need none).
   bool in_blas = false;
   bool b_last = false;    // the instance is the last of its top-level leaf
   uint32_t b_pos = 0;     // instance record whose BLAS is walked
@@ -669,10 +570,9 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
   bool b_fast = false;
   float b_limit = 0.f, b_cut = 0.f, b_t = 0.f;
   uint32_t b_best = kNoHit, b_flag = 0u;
-  float b_n[3] = {0.f, 0.f, 0.f};
   auto unified = [&]() { return IK == kInstMesh && L.kind <= kTRayCross; };
 
-  // blas_nearest's box test and leaf, on the lane's BLAS state.
+  // The box test and the leaf of a BLAS walk, on the lane's BLAS state.
   auto btest = [&](const float* lo, const float* hi, float& te) -> bool {
     int ax;
     const bool geo = b_fast ? slab_fast<3>(b_r, lo, hi, kInf, te) : slab<3>(b_r, lo, hi, kInf, te, ax);
@@ -685,11 +585,11 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
       load_vec<kBlasPrimVec>(p.bprims + size_t(pos) * kBlasPrimVec, rec);
       const uint32_t idw = __float_as_uint(rec[9]);
       const uint32_t id = idw & ~kLeafBit;
-      float t, nrm[3];
+      float t;
       if (ray_triangle(b_r.o, b_r.d, rec, rec + 3, rec + 6, t) && !(t > b_limit)) {
         if (b_best == kNoHit || hit_before(t, id, b_t, b_best)) {
-          tri_normal(rec, rec + 3, rec + 6, nrm);
           b_best = id;
+          b_tri = pos;
           b_t = t;
           b_limit = t;
           b_cut = t;
@@ -703,9 +603,6 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
             b_flag = uint32_t(t < te);
             b_cut = near_limit(t, p.window);
           }
-          b_n[0] = nrm[0];
-          b_n[1] = nrm[1];
-          b_n[2] = nrm[2];
         }
       }
       if (idw & kLeafBit) break;
@@ -782,7 +679,7 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
     return false;
   };
   // The BLAS is exhausted: its nearest hit, scaled and rotated back to
-  // world space, is the instance's hit (as after blas_nearest in leaf()).
+  // world space, is the instance's hit.
   auto blas_finish = [&]() {
     in_blas = false;
     if constexpr (IK == kInstMesh) {
@@ -791,112 +688,137 @@ __global__ void __launch_bounds__(kThreads, (IK == kInstMesh && !REF && !STATS) 
       load_vec<IL::vec>(p.insts + size_t(b_pos) * IL::vec, rec);
       const float toi = fmul(b_t, rec[IL::param]);
       if (!(toi > L.limit)) {
-        float nw[3];
-        rotate<3>(rec + IL::rot, b_n, nw);
+        float nw[3] = {0.f, 0.f, 0.f};
+        if (!is_nearest()) {
+          float tri[kBlasPrimVec * 4], nl[3];
+          load_vec<kBlasPrimVec>(p.bprims + size_t(b_tri) * kBlasPrimVec, tri);
+          tri_normal(tri, tri + 3, tri + 6, nl);
+          rotate<3>(rec + IL::rot, nl, nw);
+        }
         if (STATS) L.v_hit += 1;
         take(toi, __float_as_uint(rec[IL::id]) & ~kLeafBit, b_best, nw, b_pos, b_flag);
       }
     }
   };
 
+  // The warp steps together, as in query_kernel: each pass does one kind of
+  // work for every lane that waits for it, the kind that most lanes wait for:
+  // one node record (of either level), the triangles of one BLAS leaf, or
+  // instance work (a finished BLAS handed back, the next instance of a
+  // top-level leaf entered, a whole leaf of a query without unified levels).
+  bool b_done = false;   // the lane's BLAS is exhausted, its hit not handed back yet
+  bool live = false;     // the lane walks a query
+  bool held = false;     // the lane's query has ended, its answer is not written yet
   bool pending = false;  // this lane's query waits to be answered again in reference order
-  uint32_t pending_g = 0;
+  bool exhausted = false;  // no query is left to take (the same for the whole warp)
+  const uint32_t warps = gridDim.x * (kThreads / 32);
+  const int width = int(min(32u, max(1u, (n_total + warps - 1) / warps)));
+  const uint32_t width_mask = width >= 32 ? FULL : (1u << width) - 1u;
+  const int refill = max(1, width * kRefill / 32);
   for (;;) {
-    const bool need = !live && !exhausted && !pending;
-    const uint32_t need_mask = __ballot_sync(FULL, need);
-    uint32_t gs = kNoHit;
-    if (need_mask) {
-      const int leader = __ffs(need_mask) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(p.counter, uint32_t(__popc(need_mask)));
-      base = __shfl_sync(FULL, base, leader);
-      if (need) {
-        const uint32_t g = base + uint32_t(__popc(need_mask & lt_mask));
-        if (g < n_total) gs = g;
-        else exhausted = true;
+    uint32_t live_mask = __ballot_sync(FULL, live);
+    if (live_mask == 0u || __popc(width_mask & ~live_mask) >= refill) {
+      if (held) {
+        finish();
+        held = false;
       }
-    }
-    bool replay = false;
-    if (pending) {
-      gs = pending_g;
-      pending = false;
-      replay = true;
-    }
-    if (gs != kNoHit) {
-      L.ref = replay;
-      in_blas = false;
-      live = start(gs);
-      if (!live) finish();
-    }
-    if (!__ballot_sync(FULL, live)) {
-      if (__all_sync(FULL, exhausted)) break;
-      continue;
-    }
-    if (live) {
-      bool done = false;
-      // Descend interior records until a leaf comes up: the top level's, or
-      // the BLAS's for a lane inside an instance (the same record layout).
-      while (!(L.code & kLeafBit)) {
-        float rec[NL::vec * 4];
-        load_vec<NL::vec>((in_blas ? p.bnodes : p.nodes) + size_t(L.code) * NL::vec, rec);
-        const uint32_t ca = __float_as_uint(rec[4 * D]);
-        const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
-        float ta, tb;
-        bool pa, pb;
-        if (IK == kInstMesh && in_blas) {
-          pa = btest(rec, rec + 3, ta);
-          pb = btest(rec + 6, rec + 9, tb);
-        } else {
-          pa = test_box(rec, rec + D, ta);
-          pb = test_box(rec + 2 * D, rec + 3 * D, tb);
-          if (STATS) L.v_nodes += 2;
-        }
-        if (pa && pb) {
-          const bool a_first = (REF || !is_nearest()) ? false : (!L.ref && ta <= tb);
-          s_code[L.sp * kThreads + tid] = a_first ? cb : ca;
-          s_t[L.sp * kThreads + tid] = a_first ? tb : ta;
-          ++L.sp;
-          L.code = a_first ? ca : cb;
-        } else if (pa) {
-          L.code = ca;
-        } else if (pb) {
-          L.code = cb;
-        } else if (!pop_level()) {
-          done = true;
-          break;
-        }
+      if (pending) {
+        pending = false;
+        L.ref = true;
+        in_blas = false;
+        live = start(L.q + (L.kind <= kTRayCross ? 0u : (L.kind <= kTCastAll ? p.n_ray : p.n_ray + p.n_cast)));
+        held = !live;
       }
-      if (unified()) {
-        if (in_blas) {
-          // `done` here: the BLAS is exhausted, not the query.
-          if (!done) {
-            blas_leaf();
-            done = !pop_level();
+      const uint32_t idle_mask = width_mask & ~__ballot_sync(FULL, live || held);
+      if (!exhausted && idle_mask) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(p.counter, uint32_t(__popc(idle_mask)));
+        base = __shfl_sync(FULL, base, 0);
+        if ((idle_mask >> lane) & 1u) {
+          const uint32_t g = base + uint32_t(__popc(idle_mask & lt_mask));
+          if (g < n_total) {
+            L.ref = false;
+            in_blas = false;
+            live = start(g);
+            held = !live;
           }
-          if (done) {
-            const bool last = b_last;
-            const uint32_t next = b_pos + 1;
+        }
+        // A batch smaller than the grid's lanes is dealt out in one round.
+        exhausted = width < 32 || base + uint32_t(__popc(idle_mask)) >= n_total;
+      }
+      live_mask = __ballot_sync(FULL, live);
+      if (live_mask == 0u) {
+        if (exhausted && !__any_sync(FULL, held)) break;
+        continue;
+      }
+    }
+    const bool at_leaf = (L.code & kLeafBit) != 0u;
+    const bool at_tris = live && IK == kInstMesh && in_blas && !b_done && at_leaf;
+    const bool at_inst = live && !at_tris && (b_done || at_leaf);
+    const int n_tris = __popc(__ballot_sync(FULL, at_tris)), n_inst = __popc(__ballot_sync(FULL, at_inst));
+    const int n_node = __popc(live_mask) - n_tris - n_inst;
+    bool more = true;  // the lane's query has something left to visit
+    if (n_tris >= n_node && n_tris >= n_inst) {
+      if (at_tris) {
+        blas_leaf();
+        b_done = !pop_level();
+      }
+    } else if (n_inst >= n_node) {
+      if (at_inst) {
+        if (unified()) {
+          uint32_t next = L.code & ~kLeafBit;
+          bool enter = true;
+          if (in_blas) {
+            next = b_pos + 1;
+            enter = !b_last;
+            b_done = false;
             blas_finish();
-            done = false;
-            if (last || !enter_from(next)) done = !pop();
           }
-        } else if (!done && !enter_from(L.code & ~kLeafBit)) {
-          done = !pop();
-        }
-      } else if (!done) {
-        leaf();
-        done = !pop();
-      }
-      if (done) {
-        live = false;
-        if (!REF && !L.ref && L.flag != 0u) {
-          // answered again in the reference order at the top of the loop
-          pending = true;
-          pending_g = L.q + (L.kind <= kTRayCross ? 0u : (L.kind <= kTCastAll ? p.n_ray : p.n_ray + p.n_cast));
-          ++replays;
+          more = (enter && enter_from(next)) || pop();
         } else {
-          finish();
+          leaf();
+          more = pop();
         }
+      }
+    } else if (live && !at_tris && !at_inst) {
+      // One interior record: the top level's, or the BLAS's for a lane inside
+      // an instance (the same record layout).
+      float rec[NL::vec * 4];
+      load_vec<NL::vec>((in_blas ? p.bnodes : p.nodes) + size_t(L.code) * NL::vec, rec);
+      const uint32_t ca = __float_as_uint(rec[4 * D]);
+      const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
+      float ta, tb;
+      bool pa, pb;
+      if (IK == kInstMesh && in_blas) {
+        pa = btest(rec, rec + 3, ta);
+        pb = btest(rec + 6, rec + 9, tb);
+      } else {
+        pa = test_box(rec, rec + D, ta);
+        pb = test_box(rec + 2 * D, rec + 3 * D, tb);
+        if (STATS) L.v_nodes += 2;
+      }
+      if (pa && pb) {
+        const bool a_first = (REF || !is_nearest()) ? false : (!L.ref && ta <= tb);
+        s_code[L.sp * kThreads + tid] = a_first ? cb : ca;
+        s_t[L.sp * kThreads + tid] = a_first ? tb : ta;
+        ++L.sp;
+        L.code = a_first ? ca : cb;
+      } else if (pa) {
+        L.code = ca;
+      } else if (pb) {
+        L.code = cb;
+      } else if (!pop_level()) {
+        if (in_blas) b_done = true;
+        else more = false;
+      }
+    }
+    if (!more) {
+      live = false;
+      if (!REF && !L.ref && L.flag != 0u) {
+        pending = true;  // answered again in the reference order at the next refill
+        ++replays;
+      } else {
+        held = true;
       }
     }
   }
