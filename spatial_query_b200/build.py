@@ -27,6 +27,10 @@ UNITS = [
     ("kernels_d3.cu", ["--fmad=false"]),
     ("kernels_d4.cu", ["--fmad=false"]),
     ("kernels_d6.cu", ["--fmad=false"]),
+    ("kernels64_d2.cu", ["--fmad=false"]),
+    ("kernels64_d3.cu", ["--fmad=false"]),
+    ("kernels64_d4.cu", ["--fmad=false"]),
+    ("kernels64_d6.cu", ["--fmad=false"]),
     ("sq_tlas.cu", ["--fmad=false"]),
     ("tlas_kernels.cu", ["--fmad=false"]),
     ("guide.cu", []),

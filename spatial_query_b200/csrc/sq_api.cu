@@ -610,7 +610,7 @@ extern "C" int32_t sq_bvh_destroy(sq_bvh* b) {
   cudaSetDevice(b->device);
   void* ptrs[] = {b->d_nodes, b->d_prims, b->d_root, b->d_layers, b->d_sub, b->d_prim_ids,
                   b->d_leaves, b->d_parents, b->d_arrivals, b->d_refit_in, b->d_nonfinite,
-                  b->d_nb64, b->d_nc64, b->d_prims64, b->d_wnodes, b->d_wsrc, b->d_qnodes};
+                  b->d_root64, b->d_wnodes, b->d_wsrc, b->d_qnodes};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete b;
@@ -1428,41 +1428,6 @@ int32_t sqi::pipelined(sq_ctx* ctx, uint32_t n, const std::function<int32_t(uint
   if (ce != cudaSuccess) return cuda_fail(ctx, "chunked host-buffer call", ce);
   if (se != cudaSuccess) return cuda_fail(ctx, "chunked host-buffer call", se);
   return SQ_OK;
-}
-
-int32_t sqi::near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, const void* ref_fn, QueryParams& p,
-                               uint32_t stack) {
-  p.window = ctx->window;
-  // The replay list holds at most every query of the batch; it grows here,
-  // outside any stream capture once a batch of this size has run.
-  const size_t need = size_t(std::max<uint32_t>(p.n, 1)) * sizeof(uint32_t);
-  if (ctx->replay_list.cap < need) {
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (ctx->replay_list.p) CK(cudaFree(ctx->replay_list.p));
-    ctx->replay_list.p = nullptr;
-    ctx->replay_list.cap = 0;
-    CK(cudaMalloc(&ctx->replay_list.p, need));
-    ctx->replay_list.cap = need;
-  }
-  CK(cudaMemsetAsync(ctx->d_replays, 0, sizeof(uint32_t), ctx->stream));
-  const bool replays = b->narrow != SQ_NARROW_AABB;
-  uint32_t* counters = nullptr;
-  int32_t rc = work_counters(ctx, replays ? 2 : 1, &counters);
-  if (rc) return rc;
-  p.replay_count = ctx->d_replays;
-  p.replay_list = static_cast<uint32_t*>(ctx->replay_list.p);
-  if ((rc = launch_persistent(ctx, fn, p, stack, p.n, counters))) return rc;
-  // A box leaf's hit is its own slab entry, so box answers are always
-  // certified and nothing is ever appended: no replay launch.
-  if (!replays) return SQ_OK;
-  // The uncertified queries again, in the reference order, unseeded.
-  QueryParams r = p;
-  r.replay_count = nullptr;
-  r.replay_list = nullptr;
-  r.seed_bucket = nullptr;
-  r.q_list = static_cast<const uint32_t*>(ctx->replay_list.p);
-  r.q_count = ctx->d_replays;
-  return launch_persistent(ctx, ref_fn, r, b->depth, p.n, counters + 1);
 }
 
 // ============================================================================

@@ -1,27 +1,19 @@
 // The crate's f64 feature on the device (Scalar = f64, maths/point.rs:14-18):
-// nearest rays against an f64 scene, for consumers whose coordinates need
-// double precision (large worlds) or who compare against an f64 CPU build.
+// queries against an f64 scene, for consumers whose coordinates need double
+// precision (large worlds) or who compare against an f64 CPU build.
 //
-// The walk is Bvh::raycast_nearest_impl (accel/bvh.rs:73-124) as written: a
-// stack of node indices seeded with the root; a popped node is tested with
-// Aabb::ray_intersect against the current limit; a leaf tests its accepted
-// primitives in prim_indices order with the limit, keeping the first hit in
-// hit_ordering and shrinking the limit to it; an interior node pushes
-// child_a then child_b. All arithmetic is the f64 form of the f32 kernels'
-// (sq_math.cuh with S = double), so answers and QueryStats counters equal the
-// f64 CPU path's bit for bit. One thread per ray; the node boxes and links
-// are the host tree's nodes as they are (no child-pair records).
-//
-// The crate's other queries take the same walk on f64 scenes (walk64_kernel):
-// raycast_all and raycast_crossings (bvh.rs:196-328: no limit shrink, hits
-// kept in hit_ordering, bounded to k per ray with the full count),
-// shapecast_nearest / shapecast_all (bvh.rs:330-414: the node test is
-// ShapeCast::broadphase, the slab against the box grown by the probe) and
-// overlap (bvh.rs:416-456: Aabb::intersects per node, CSR output with each
-// region's leaves ascending).
+// The kernels are query_kernel's with S = double (traverse.cuh): child-pair
+// records of doubles, nearest queries near-first with the certificate (or in
+// the crate's own order, which the counters ask for: Bvh::raycast_nearest_impl,
+// accel/bvh.rs:73-124), lists, casts and overlap in the crate's order
+// (bvh.rs:196-456). All arithmetic is the f64 form of the f32 kernels'
+// (sq_math.cuh), so answers and QueryStats counters equal the f64 CPU path's
+// bit for bit.
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <memory>
 #include <string>
 #include <vector>
@@ -34,405 +26,39 @@ using sqi::fail;
 
 namespace {
 
-constexpr int kStack64 = kMaxStack;  // deepest tree accepted, as for f32 scenes
+using namespace sqi;
+using Params64 = QueryParamsT<double>;
 
-struct Params64 {
-  const double* nb;    // [n_nodes][2D]
-  const uint2* nc;     // [n_nodes]
-  const double* prims; // [n_prims][stride], leaf order
-  const uint32_t* ids; // [n_prims]: leaf id at each position
-  const uint64_t* layers;
-  uint64_t mask;
-  long long exclude;
-  uint32_t stride;
-  const double* rays;  // [n][2D]
-  uint32_t n;
-  double max_toi;
-  const double* max_toi_arr;
-  uint32_t* out_leaf;
-  double* out_toi;
-  double* out_normal;
-  unsigned long long* stats;  // nodes, aabb tests, narrow tests, hits (summed)
-  // walk64_kernel: queries (rays o,d; casts o,d,probe.min,probe.max; regions lo,hi)
-  uint32_t k;                 // list capacity per query
-  int crossings;              // raycast_crossings: both roots of sphere leaves
-  uint32_t* out_count;        // lists: full count; overlap count pass: results per region
-  const unsigned long long* csr_offsets;  // overlap fill pass
-  uint32_t* csr_leaves;
-};
-
-template <int D, int N>
-__device__ __forceinline__ bool narrow64(const double* rec, const RayPre<D, double>& r, double limit, double& t,
-                                         double* n) {
-  if constexpr (N == kNarrowAabb) {
-    int axis;
-    if (!slab<D>(r, rec, rec + D, limit, t, axis)) return false;
-    entry_normal<D>(r.d, axis, n);
-    return true;
-  } else if constexpr (N == kNarrowSphere || N == kNarrowSphereNear) {
-    return ray_ball<D, N == kNarrowSphere>(r.o, r.d, rec, rec[D], limit, t, n);
-  } else {
-    if (!ray_triangle(r.o, r.d, rec, rec + 3, rec + 6, t)) return false;
-    if (t > limit) return false;
-    tri_normal(rec, rec + 3, rec + 6, n);
-    return true;
-  }
-}
-
-template <int D, int N, bool STATS>
-__global__ void __launch_bounds__(128) nearest64_kernel(const Params64 p) {
-  unsigned long long c_nodes = 0, c_nar = 0, c_hit = 0;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < p.n; q += gridDim.x * blockDim.x) {
-    RayPre<D, double> r;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      r.o[i] = p.rays[size_t(q) * 2 * D + i];
-      r.d[i] = p.rays[size_t(q) * 2 * D + D + i];
-    }
-    ray_prep(r);
-    double limit = p.max_toi_arr ? p.max_toi_arr[q] : p.max_toi;
-    uint32_t best = kNoHit;
-    double best_t = 0.0, best_n[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) best_n[i] = 0.0;
-    uint32_t stack[kStack64];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-      const uint32_t ni = stack[--sp];
-      if (STATS) ++c_nodes;
-      double te;
-      int ax;
-      const double* nb = p.nb + size_t(ni) * 2 * D;
-      if (!slab<D>(r, nb, nb + D, limit, te, ax) || !(te <= limit)) continue;
-      const uint2 c = p.nc[ni];
-      if (c.y & kLeafBit) {
-        const uint32_t end = c.x + (c.y & ~kLeafBit);
-        for (uint32_t pos = c.x; pos < end; ++pos) {
-          const uint32_t id = p.ids[pos];
-          if (p.layers && ((p.exclude >= 0 && (unsigned long long)p.exclude == id) || !(p.layers[id] & p.mask)))
-            continue;
-          if (STATS) ++c_nar;
-          double t, nrm[D];
-          if (narrow64<D, N>(p.prims + size_t(pos) * p.stride, r, limit, t, nrm)) {
-            if (STATS) ++c_hit;
-            if (best == kNoHit || hit_before(t, id, best_t, best)) {
-              best = id;
-              best_t = t;
-              limit = t;
-#pragma unroll
-              for (int i = 0; i < D; ++i) best_n[i] = nrm[i];
-            }
-          }
-        }
-      } else if (sp + 2 <= kStack64) {  // the upload bounds the depth, so this always holds
-        stack[sp++] = c.x;
-        stack[sp++] = c.y;
-      }
-    }
-    p.out_leaf[q] = best;
-    if (p.out_toi) p.out_toi[q] = best_t;
-    if (p.out_normal) {
-#pragma unroll
-      for (int i = 0; i < D; ++i) p.out_normal[size_t(q) * D + i] = best_n[i];
-    }
-  }
-  if (STATS && p.stats) {
-    atomicAdd(p.stats + 0, c_nodes);
-    atomicAdd(p.stats + 1, c_nodes);  // one box test per visited node (bvh.rs:91-92)
-    atomicAdd(p.stats + 2, c_nar);
-    atomicAdd(p.stats + 3, c_hit);
-  }
-}
-
-// One primitive's swept-probe test (QueryGeometry::test_shape_cast of the
-// built-in providers, as the f32 kernels answer it): boxes the grown slab,
-// balls the ray against the ball grown by probe.max[0], triangles the grown
-// slab against the triangle's AABB.
-template <int D, int N>
-__device__ __forceinline__ bool cast64(const double* rec, const RayPre<D, double>& r, const double* pmin,
-                                       const double* pmax, double limit, double& t, double* n) {
-  if constexpr (N == kNarrowAabb) {
-    int axis;
-    if (!slab_grown<D>(r, rec, rec + D, pmin, pmax, limit, t, axis)) return false;
-    entry_normal<D>(r.d, axis, n);
-    return true;
-  } else if constexpr (N == kNarrowSphere || N == kNarrowSphereNear) {
-    return ray_ball<D, N == kNarrowSphere>(r.o, r.d, rec, sq::fadd(rec[D], pmax[0]), limit, t, n);
-  } else {
-    double lo[3], hi[3];
-    tri_aabb(rec, rec + 3, rec + 6, lo, hi);
-    int axis;
-    if (!slab_grown<3>(r, lo, hi, pmin, pmax, limit, t, axis)) return false;
-    entry_normal<3>(r.d, axis, n);
-    return true;
-  }
-}
-
-// One primitive's overlap test (QueryGeometry::test_overlap).
-template <int D, int N>
-__device__ __forceinline__ bool overlap64(const double* rec, const double* qlo, const double* qhi) {
-  if constexpr (N == kNarrowAabb) {
-    return box_overlap<D>(rec, rec + D, qlo, qhi);
-  } else if constexpr (N == kNarrowSphere || N == kNarrowSphereNear) {
-    double d2 = 0.0;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      const double c = rec[i];
-      const double v = (c < qlo[i]) ? sq::fsub(qlo[i], c) : ((c > qhi[i]) ? sq::fsub(c, qhi[i]) : 0.0);
-      d2 = sq::fadd(d2, sq::fmul(v, v));
-    }
-    return sq::fsqrt(d2) <= rec[D];
-  } else {
-    double lo[3], hi[3];
-    tri_aabb(rec, rec + 3, rec + 6, lo, hi);
-    return box_overlap<3>(lo, hi, qlo, qhi);
-  }
-}
-
-// Sorted insertion into query q's bounded list (hit_ordering; an equal key
-// goes after the entries already there). `count` is the full number so far.
-template <int D>
-__device__ __forceinline__ void put64(const Params64& p, uint32_t q, uint32_t& count, double t, uint32_t leaf,
-                                      const double* n) {
-  uint32_t m = count < p.k ? count : p.k;
-  ++count;
-  if (p.k == 0) return;
-  const size_t base = size_t(q) * p.k;
-  uint32_t* ol = p.out_leaf;
-  double* ot = p.out_toi;
-  double* on = p.out_normal;
-  if (m == p.k) {
-    if (!hit_before(t, leaf, ot[base + p.k - 1], ol[base + p.k - 1])) return;
-    m = p.k - 1;
-  }
-  uint32_t j = m;
-  while (j > 0 && hit_before(t, leaf, ot[base + j - 1], ol[base + j - 1])) {
-    ot[base + j] = ot[base + j - 1];
-    ol[base + j] = ol[base + j - 1];
-    if (on)
-#pragma unroll
-      for (int i = 0; i < D; ++i) on[(base + j) * D + i] = on[(base + j - 1) * D + i];
-    --j;
-  }
-  ot[base + j] = t;
-  ol[base + j] = leaf;
-  if (on)
-#pragma unroll
-    for (int i = 0; i < D; ++i) on[(base + j) * D + i] = n[i];
-}
-
-// The crate's walk (push child_a, push child_b; pop, test the node against
-// the query, open a leaf) for lists, casts and overlap on an f64 scene.
-// K: kRayAll (p.crossings: raycast_crossings), kCastNearest, kCastAll,
-// kOverlap (p.csr_leaves null: count pass; else fill in walk order).
-template <int D, int N, int K>
-__global__ void __launch_bounds__(128) walk64_kernel(const Params64 p) {
-  constexpr bool kCast = (K == kCastNearest || K == kCastAll);
-  constexpr int QW = kCast ? 4 * D : 2 * D;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < p.n; q += gridDim.x * blockDim.x) {
-    const double* src = p.rays + size_t(q) * QW;
-    RayPre<D, double> r;
-    double pmin[D], pmax[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      r.o[i] = src[i];
-      r.d[i] = src[D + i];
-      if constexpr (kCast) {
-        pmin[i] = src[2 * D + i];
-        pmax[i] = src[3 * D + i];
-      } else {
-        pmin[i] = pmax[i] = 0.0;
-      }
-    }
-    if constexpr (K != kOverlap) ray_prep(r);
-    double limit = p.max_toi_arr ? p.max_toi_arr[q] : p.max_toi;
-    uint32_t best = kNoHit, count = 0;
-    double best_t = 0.0, best_n[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) best_n[i] = 0.0;
-    const unsigned long long csr_base = (K == kOverlap && p.csr_leaves) ? p.csr_offsets[q] : 0ull;
-    uint32_t stack[kStack64];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-      const uint32_t ni = stack[--sp];
-      const double* nb = p.nb + size_t(ni) * 2 * D;
-      if constexpr (K == kOverlap) {
-        if (!box_overlap<D>(nb, nb + D, r.o, r.d)) continue;  // region lo / hi sit in o / d
-      } else {
-        double te;
-        int ax;
-        bool geo;
-        if constexpr (kCast) geo = slab_grown<D>(r, nb, nb + D, pmin, pmax, limit, te, ax);
-        else geo = slab<D>(r, nb, nb + D, limit, te, ax);
-        if (!geo || !(te <= limit)) continue;
-      }
-      const uint2 c = p.nc[ni];
-      if (!(c.y & kLeafBit)) {
-        if (sp + 2 <= kStack64) {  // the upload bounds the depth, so this always holds
-          stack[sp++] = c.x;
-          stack[sp++] = c.y;
-        }
-        continue;
-      }
-      const uint32_t end = c.x + (c.y & ~kLeafBit);
-      for (uint32_t pos = c.x; pos < end; ++pos) {
-        const uint32_t id = p.ids[pos];
-        if (p.layers && ((p.exclude >= 0 && (unsigned long long)p.exclude == id) || !(p.layers[id] & p.mask)))
-          continue;
-        const double* rec = p.prims + size_t(pos) * p.stride;
-        double t, nrm[D];
-        if constexpr (K == kOverlap) {
-          if (overlap64<D, N>(rec, r.o, r.d)) {
-            if (p.csr_leaves) p.csr_leaves[csr_base + count] = id;
-            ++count;
-          }
-        } else if constexpr (K == kCastNearest) {
-          if (cast64<D, N>(rec, r, pmin, pmax, limit, t, nrm) &&
-              (best == kNoHit || hit_before(t, id, best_t, best))) {
-            best = id;
-            best_t = t;
-            limit = t;
-#pragma unroll
-            for (int i = 0; i < D; ++i) best_n[i] = nrm[i];
-          }
-        } else if constexpr (K == kCastAll) {
-          if (cast64<D, N>(rec, r, pmin, pmax, limit, t, nrm)) put64<D>(p, q, count, t, id, nrm);
-        } else {  // kRayAll
-          bool listed = false;
-          // Both roots for the ball whose test reports the far root from
-          // inside (tests/crossings.rs:505-521); the near-root-only ball lists
-          // one crossing per hit, as the f32 kernels do.
-          if constexpr (N == kNarrowSphere) {
-            if (p.crossings) {
-              // Both roots of the unbounded ray (tests/crossings.rs:505-521).
-              listed = true;
-              double oc[D];
-#pragma unroll
-              for (int i = 0; i < D; ++i) oc[i] = sq::fsub(r.o[i], rec[i]);
-              const double b = pdot<D>(oc, r.d);
-              const double disc = sq::fsub(sq::fmul(b, b), sq::fsub(pdot<D>(oc, oc), sq::fmul(rec[D], rec[D])));
-              if (!(disc < 0.0)) {
-                const double sq = sq::fsqrt(disc);
-                const double roots[2] = {sq::fsub(-b, sq), sq::fadd(-b, sq)};
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                  const double tt = roots[j];
-                  if (tt >= 0.0 && tt <= limit) {
-                    double pt[D];
-                    ray_at<D>(r.o, r.d, tt, pt);
-#pragma unroll
-                    for (int i = 0; i < D; ++i) nrm[i] = sq::fsub(pt[i], rec[i]);
-                    normalize_or_zero<D>(nrm);
-                    put64<D>(p, q, count, tt, id, nrm);
-                  }
-                }
-              }
-            }
-          }
-          if (!listed && narrow64<D, N>(rec, r, limit, t, nrm)) put64<D>(p, q, count, t, id, nrm);
-        }
-      }
-    }
-    if constexpr (K == kCastNearest) {
-      p.out_leaf[q] = best;
-      if (p.out_toi) p.out_toi[q] = best_t;
-      if (p.out_normal) {
-#pragma unroll
-        for (int i = 0; i < D; ++i) p.out_normal[size_t(q) * D + i] = best_n[i];
-      }
-    } else if constexpr (K == kOverlap) {
-      if (!p.csr_leaves) p.out_count[q] = count;
-    } else {
-      p.out_count[q] = count;
-    }
-  }
-}
-
-template <int D, int N>
-const void* pick(bool stats) {
-  return stats ? reinterpret_cast<const void*>(&nearest64_kernel<D, N, true>)
-               : reinterpret_cast<const void*>(&nearest64_kernel<D, N, false>);
-}
-
-template <int D>
-const void* pick_narrow(int narrow, bool stats) {
-  switch (narrow) {
-    case SQ_NARROW_AABB: return pick<D, kNarrowAabb>(stats);
-    case SQ_NARROW_SPHERE: return pick<D, kNarrowSphere>(stats);
-    case SQ_NARROW_SPHERE_NEAR: return pick<D, kNarrowSphereNear>(stats);
-    case SQ_NARROW_TRIANGLE:
-      if constexpr (D == 3) return pick<3, kNarrowTri>(stats);
-      return nullptr;
-    default: return nullptr;
-  }
-}
-
-const void* kernel64(int dim, int narrow, bool stats) {
+bool kernel_set64(int dim, int narrow, KernelSet* out) {
   switch (dim) {
-    case 2: return pick_narrow<2>(narrow, stats);
-    case 3: return pick_narrow<3>(narrow, stats);
-    case 4: return pick_narrow<4>(narrow, stats);
-    case 6: return pick_narrow<6>(narrow, stats);
-    default: return nullptr;
-  }
-}
-
-template <int D, int N>
-const void* walk_pick(int kind) {
-  switch (kind) {
-    case kRayAll: return reinterpret_cast<const void*>(&walk64_kernel<D, N, kRayAll>);
-    case kCastNearest: return reinterpret_cast<const void*>(&walk64_kernel<D, N, kCastNearest>);
-    case kCastAll: return reinterpret_cast<const void*>(&walk64_kernel<D, N, kCastAll>);
-    case kOverlap: return reinterpret_cast<const void*>(&walk64_kernel<D, N, kOverlap>);
-    default: return nullptr;
-  }
-}
-
-template <int D>
-const void* walk_narrow(int narrow, int kind) {
-  switch (narrow) {
-    case SQ_NARROW_AABB: return walk_pick<D, kNarrowAabb>(kind);
-    case SQ_NARROW_SPHERE: return walk_pick<D, kNarrowSphere>(kind);
-    case SQ_NARROW_SPHERE_NEAR: return walk_pick<D, kNarrowSphereNear>(kind);
-    case SQ_NARROW_TRIANGLE:
-      if constexpr (D == 3) return walk_pick<3, kNarrowTri>(kind);
-      return nullptr;
-    default: return nullptr;
-  }
-}
-
-const void* walk64(int dim, int narrow, int kind) {
-  switch (dim) {
-    case 2: return walk_narrow<2>(narrow, kind);
-    case 3: return walk_narrow<3>(narrow, kind);
-    case 4: return walk_narrow<4>(narrow, kind);
-    case 6: return walk_narrow<6>(narrow, kind);
-    default: return nullptr;
+    case 2: return kernel_set64_d2(narrow, out);
+    case 3: return kernel_set64_d3(narrow, out);
+    case 4: return kernel_set64_d4(narrow, out);
+    case 6: return kernel_set64_d6(narrow, out);
+    default: return false;
   }
 }
 
 Params64 base64(const sq_bvh* b, const sq_filter* filter) {
   Params64 p{};
-  p.nb = b->d_nb64;
-  p.nc = b->d_nc64;
-  p.prims = b->d_prims64;
-  p.ids = b->d_prim_ids;
+  p.nodes = b->d_nodes;
+  p.prims = b->d_prims;
   p.layers = b->d_layers;
+  p.root_box = b->d_root64;
+  p.nonfinite = b->d_nonfinite;
+  p.root_code = b->root_code;
   p.mask = filter ? filter->layer_mask : ~0ull;
   p.exclude = filter ? filter->exclude : -1;
-  p.stride = b->stride;
   return p;
 }
 
-int32_t launch64(sq_ctx* ctx, const void* fn, Params64& p) {
-  if (!fn) return fail(ctx, SQ_ERR_UNSUPPORTED, "no f64 kernel for this scene");
-  const uint32_t grid = std::min<uint32_t>((p.n + 127) / 128, uint32_t(ctx->sm_count) * 16);
-  void* args[] = {&p};
-  CK(cudaLaunchKernel(fn, dim3(std::max<uint32_t>(grid, 1)), dim3(128), args, 0, ctx->stream));
-  ctx->launches++;
-  return SQ_OK;
+// Nearest rays (counted: stats) or casts: near-first with the certificate, or
+// the crate's own order when the context asks for it and for counters, which
+// are the crate's.
+int32_t nearest64(sq_ctx* ctx, const sq_bvh* b, bool cast, Params64& p, bool stats) {
+  const void* ref_fn = cast ? b->ks64.cast_nearest[1] : b->ks64.ray_nearest[1][stats ? 1 : 0];
+  if (stats || ctx->order == SQ_ORDER_REFERENCE) return launch_persistent(ctx, ref_fn, p, b->depth, p.n);
+  return near_first_launch(ctx, b, cast ? b->ks64.cast_nearest[0] : b->ks64.ray_nearest[0][0], ref_fn, p, b->depth);
 }
 
 uint32_t stride64(int dim, int narrow) {
@@ -460,7 +86,8 @@ extern "C" int32_t sq_bvh_upload_f64(sq_ctx* ctx, int32_t dim, int32_t narrow, u
                                      sq_bvh** out) {
   if (!ctx || !out) return SQ_ERR_INVALID;
   *out = nullptr;
-  if (!kernel64(dim, narrow, false))
+  KernelSet ks;
+  if (!kernel_set64(dim, narrow, &ks))
     return fail(ctx, SQ_ERR_UNSUPPORTED, "no f64 kernels for dim " + std::to_string(dim) + " narrow " +
                                              std::to_string(narrow));
   if (prim_stride != stride64(dim, narrow)) return fail(ctx, SQ_ERR_INVALID, "prim_stride does not match the narrow phase");
@@ -477,6 +104,7 @@ extern "C" int32_t sq_bvh_upload_f64(sq_ctx* ctx, int32_t dim, int32_t narrow, u
   b->n_nodes = n_nodes;
   b->n_prims = n_prims;
   b->stride = prim_stride;
+  b->ks64 = ks;
   if (n_nodes == 0) {
     *out = b.release();
     return SQ_OK;
@@ -494,7 +122,7 @@ extern "C" int32_t sq_bvh_upload_f64(sq_ctx* ctx, int32_t dim, int32_t narrow, u
     }
   }
   b->depth = depth[0];
-  if (b->depth + 1 > uint32_t(kStack64))
+  if (b->depth + 1 > uint32_t(kMaxStack))
     return fail(ctx, SQ_ERR_DEPTH, "tree depth " + std::to_string(b->depth) + " exceeds the traversal stack");
   {
     std::vector<uint8_t> seen(n_prims, 0), covered(n_prims, 0);
@@ -513,12 +141,37 @@ extern "C" int32_t sq_bvh_upload_f64(sq_ctx* ctx, int32_t dim, int32_t narrow, u
     for (uint32_t k = 0; k < n_prims; ++k)
       if (!covered[k]) return fail(ctx, SQ_ERR_INVALID, "leaf ranges leave a primitive uncovered");
   }
-  std::vector<uint2> links(n_nodes);
+  // Child-pair node records and leaf-ordered primitive records, as the f32
+  // upload lays them out: the boxes in doubles, then both codes in one 8-byte
+  // word; the parameters in doubles, then the id word in the low half of one.
+  const int D = dim;
+  std::vector<uint32_t> iidx(n_nodes, kNoHit);
   for (uint32_t i = 0; i < n_nodes; ++i)
-    links[i] = prim_count[i] == 0 ? make_uint2(child_a[i], child_b[i]) : make_uint2(child_a[i], prim_count[i] | kLeafBit);
-  std::vector<double> prims(size_t(n_prims) * prim_stride);
-  for (uint32_t pos = 0; pos < n_prims; ++pos)
-    std::copy_n(prim_data + size_t(prim_indices[pos]) * prim_stride, prim_stride, prims.data() + size_t(pos) * prim_stride);
+    if (prim_count[i] == 0) iidx[i] = b->n_interior++;
+  auto code = [&](uint32_t i) { return prim_count[i] == 0 ? iidx[i] : (kLeafBit | child_a[i]); };
+  b->root_code = code(0);
+  const size_t NS = size_t(record_vec(8 * D + 2)) * 2, PS = size_t(record_vec(2 * (int(prim_stride) + 1))) * 2;
+  b->prim_vec = uint32_t(PS / 2);
+  std::vector<double> nodes(std::max<size_t>(b->n_interior, 1) * NS, 0.0), prims(size_t(n_prims) * PS, 0.0);
+  for (uint32_t i = 0; i < n_nodes; ++i) {
+    if (prim_count[i] == 0) {
+      double* r = nodes.data() + size_t(iidx[i]) * NS;
+      const uint32_t ch[2] = {child_a[i], child_b[i]}, codes[2] = {code(child_a[i]), code(child_b[i])};
+      for (int s = 0; s < 2; ++s) std::copy_n(node_bounds + size_t(ch[s]) * 2 * D, 2 * D, r + s * 2 * D);
+      std::memcpy(r + 4 * D, codes, sizeof(codes));
+      continue;
+    }
+    for (uint32_t j = 0; j < prim_count[i]; ++j) {
+      const uint32_t pos = child_a[i] + j, id = prim_indices[pos];
+      double* r = prims.data() + size_t(pos) * PS;
+      std::copy_n(prim_data + size_t(id) * prim_stride, prim_stride, r);
+      const uint64_t w = id | (j + 1 == prim_count[i] ? kLeafBit : 0u);
+      std::memcpy(r + prim_stride, &w, sizeof(w));
+    }
+  }
+  int nonfinite = 0;
+  for (size_t k = 0; k < size_t(n_nodes) * 2 * D; ++k)
+    if (!std::isfinite(node_bounds[k])) nonfinite = 1;
   auto up = [&](void** dst, const void* src, size_t bytes) -> int32_t {
     CK(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
     if (src && bytes) CK(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
@@ -530,10 +183,10 @@ extern "C" int32_t sq_bvh_upload_f64(sq_ctx* ctx, int32_t dim, int32_t narrow, u
     sq_bvh_destroy(b.release());
     return code;
   };
-  if ((rc = up((void**)&b->d_nb64, node_bounds, size_t(n_nodes) * 2 * dim * 8))) return cleanup(rc);
-  if ((rc = up((void**)&b->d_nc64, links.data(), links.size() * sizeof(uint2)))) return cleanup(rc);
-  if ((rc = up((void**)&b->d_prims64, prims.data(), prims.size() * 8))) return cleanup(rc);
-  if ((rc = up((void**)&b->d_prim_ids, prim_indices, size_t(n_prims) * 4))) return cleanup(rc);
+  if ((rc = up((void**)&b->d_nodes, nodes.data(), nodes.size() * 8))) return cleanup(rc);
+  if ((rc = up((void**)&b->d_prims, prims.data(), prims.size() * 8))) return cleanup(rc);
+  if ((rc = up((void**)&b->d_root64, node_bounds, size_t(2) * D * 8))) return cleanup(rc);
+  if ((rc = up((void**)&b->d_nonfinite, &nonfinite, sizeof(int)))) return cleanup(rc);
   if (layers && (rc = up((void**)&b->d_layers, layers, size_t(n_prims) * 8))) return cleanup(rc);
   *out = b.release();
   return SQ_OK;
@@ -554,16 +207,8 @@ extern "C" int32_t sq_raycast_nearest_f64_d(sq_ctx* ctx, const sq_bvh* b, const 
     if (d_toi) CK(cudaMemsetAsync(d_toi, 0, size_t(n) * 8, ctx->stream));
     if (d_normal) CK(cudaMemsetAsync(d_normal, 0, size_t(n) * b->dim * 8, ctx->stream));
   } else {
-    Params64 p{};
-    p.nb = b->d_nb64;
-    p.nc = b->d_nc64;
-    p.prims = b->d_prims64;
-    p.ids = b->d_prim_ids;
-    p.layers = b->d_layers;
-    p.mask = filter ? filter->layer_mask : ~0ull;
-    p.exclude = filter ? filter->exclude : -1;
-    p.stride = b->stride;
-    p.rays = d_rays;
+    Params64 p = base64(b, filter);
+    p.queries = d_rays;
     p.n = n;
     p.max_toi = max_toi;
     p.max_toi_arr = d_max_toi_per_query;
@@ -571,11 +216,7 @@ extern "C" int32_t sq_raycast_nearest_f64_d(sq_ctx* ctx, const sq_bvh* b, const 
     p.out_toi = d_toi;
     p.out_normal = d_normal;
     p.stats = st ? ctx->d_stats : nullptr;
-    const void* fn = kernel64(b->dim, b->narrow, st);
-    const uint32_t grid = std::min<uint32_t>((n + 127) / 128, uint32_t(ctx->sm_count) * 16);
-    void* args[] = {&p};
-    CK(cudaLaunchKernel(fn, dim3(grid), dim3(128), args, 0, ctx->stream));
-    ctx->launches++;
+    if ((rc = nearest64(ctx, b, false, p, st))) return rc;
   }
   CK(cudaGetLastError());
   if (st) {
@@ -643,7 +284,7 @@ int32_t lists64(sq_ctx* ctx, const sq_bvh* b, int kind, const double* d_q, uint3
     return SQ_OK;
   }
   Params64 p = base64(b, filter);
-  p.rays = d_q;
+  p.queries = d_q;
   p.n = n;
   p.max_toi = max_toi;
   p.max_toi_arr = d_mt;
@@ -653,7 +294,7 @@ int32_t lists64(sq_ctx* ctx, const sq_bvh* b, int kind, const double* d_q, uint3
   p.out_leaf = o->leaf;
   p.out_toi = o->toi;
   p.out_normal = o->normal;
-  return launch64(ctx, walk64(b->dim, b->narrow, kind), p);
+  return launch_persistent(ctx, kind == kCastAll ? b->ks64.cast_all : b->ks64.ray_all[0], p, b->depth, p.n);
 }
 
 // Host-buffer lists: queries (and per-query limits) in, lists out, through
@@ -738,14 +379,14 @@ extern "C" int32_t sq_shapecast_nearest_f64_d(sq_ctx* ctx, const sq_bvh* b, cons
     return SQ_OK;
   }
   Params64 p = base64(b, filter);
-  p.rays = d_casts;
+  p.queries = d_casts;
   p.n = n;
   p.max_toi = max_toi;
   p.max_toi_arr = d_max_toi_per_query;
   p.out_leaf = d_leaf;
   p.out_toi = d_toi;
   p.out_normal = d_normal;
-  return launch64(ctx, walk64(b->dim, b->narrow, kCastNearest), p);
+  return nearest64(ctx, b, true, p, false);
 }
 
 extern "C" int32_t sq_shapecast_nearest_f64(sq_ctx* ctx, const sq_bvh* b, const double* casts, uint32_t n,
@@ -796,11 +437,11 @@ extern "C" int32_t sq_overlap_f64_d(sq_ctx* ctx, const sq_bvh* b, const double* 
   uint32_t* d_counts = reinterpret_cast<uint32_t*>(base + o_cnt);
   CK(cudaMemsetAsync(d_counts, 0, (size_t(n) + 1) * 4, ctx->stream));
   Params64 p = base64(b, filter);
-  p.rays = d_regions;
+  p.queries = d_regions;
   p.n = n;
   p.out_count = d_counts;
-  const void* fn = walk64(b->dim, b->narrow, kOverlap);
-  if (b->n_nodes != 0 && n != 0 && (rc = launch64(ctx, fn, p))) return rc;
+  const void* fn = b->ks64.overlap;
+  if (b->n_nodes != 0 && n != 0 && (rc = launch_persistent(ctx, fn, p, b->depth, p.n))) return rc;
   CK(cub::DeviceScan::ExclusiveScan(base + o_tmp, scan_bytes, d_counts, reinterpret_cast<unsigned long long*>(d_offsets),
                                     cuda::std::plus<>{}, 0ull, int(n) + 1, ctx->stream));
   ctx->launches++;
@@ -813,7 +454,8 @@ extern "C" int32_t sq_overlap_f64_d(sq_ctx* ctx, const sq_bvh* b, const double* 
     if (!d_leaves) return fail(ctx, SQ_ERR_INVALID, "null leaf output");
     p.csr_offsets = reinterpret_cast<const unsigned long long*>(d_offsets);
     p.csr_leaves = d_leaves;
-    if ((rc = launch64(ctx, fn, p))) return rc;
+    p.fill = 2;
+    if ((rc = launch_persistent(ctx, fn, p, b->depth, p.n))) return rc;
     if ((rc = sqi::sort_csr_segments(ctx, d_leaves, tot, d_offsets, n))) return rc;
   }
   CK(cudaStreamSynchronize(ctx->stream));

@@ -20,6 +20,11 @@ bool kernel_set_d2(int narrow, KernelSet* out);
 bool kernel_set_d3(int narrow, KernelSet* out);
 bool kernel_set_d4(int narrow, KernelSet* out);
 bool kernel_set_d6(int narrow, KernelSet* out);
+// The kernels of f64 scenes.
+bool kernel_set64_d2(int narrow, KernelSet* out);
+bool kernel_set64_d3(int narrow, KernelSet* out);
+bool kernel_set64_d4(int narrow, KernelSet* out);
+bool kernel_set64_d6(int narrow, KernelSet* out);
 }  // namespace sq
 
 
@@ -90,22 +95,17 @@ struct sq_bvh {
   uint32_t n_wide = 0, wroot = 0, wdepth = 0;
   // The same four-wide records quantised (QuantLayout), same numbering.
   float4* d_qnodes = nullptr;
-  // An f64 scene (sq_bvh_upload_f64): node boxes, node links and leaf
-  // parameters in double, answered only by the _f64 entry points.
+  // An f64 scene (sq_bvh_upload_f64): d_nodes and d_prims hold f64 records,
+  // d_root64 the root box, and only the _f64 entry points answer it, through
+  // ks64 (ks stays empty, so that no f32 call finds a kernel).
   int prec = 32;
-  double* d_nb64 = nullptr;   // [n_nodes][2D]
-  uint2* d_nc64 = nullptr;    // [n_nodes]: (child_a, child_b), or (first, count | kLeafBit)
-  double* d_prims64 = nullptr;  // [n_prims][stride], leaf order
+  double* d_root64 = nullptr;
+  sq::KernelSet ks64{};
 };
 
 namespace sqi {
 
 using namespace sq;
-
-// Near-first nearest launch `fn` followed by the reference-order replay
-// (`ref_fn`) of the queries it could not certify (sq_api.cu).
-int32_t near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, const void* ref_fn, QueryParams& p,
-                          uint32_t stack);
 
 // Consumer narrow phases (rtc.cpp): the kernels of a D = 3 scene whose
 // narrow phase is `src` with `stride` floats per leaf, compiled with NVRTC
@@ -265,7 +265,7 @@ inline int32_t launch_persistent(sq_ctx* ctx, const void* fn, Params& p, uint32_
   }
   p.counter = ctr;
   p.stack = int(std::max<uint32_t>(depth, 1));
-  const size_t smem = size_t(p.stack) * kThreads * 8;
+  const size_t smem = size_t(p.stack) * kThreads * Params::kEntryBytes;
   if (smem > 48 * 1024) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   int bps = ctx->blocks_per_sm > 0 ? ctx->blocks_per_sm : occupancy(ctx, fn, smem);
   // A warp takes at most its share of the queries (query_kernel's width): a
@@ -278,5 +278,49 @@ inline int32_t launch_persistent(sq_ctx* ctx, const void* fn, Params& p, uint32_
   return SQ_OK;
 }
 
+// Near-first nearest launch `fn` followed by the reference-order replay
+// (`ref_fn`) of the queries it could not certify.
+template <class S>
+inline int32_t near_first_launch(sq_ctx* ctx, const sq_bvh* b, const void* fn, const void* ref_fn, QueryParamsT<S>& p,
+                                 uint32_t stack) {
+  p.window = ctx->window;
+  // The replay list holds at most every query of the batch; it grows here,
+  // outside any stream capture once a batch of this size has run. An f64 call
+  // needed no scratch before it had this list: while a capture is under way
+  // that it cannot grow in, such a call is answered in the reference order.
+  const size_t need = size_t(std::max<uint32_t>(p.n, 1)) * sizeof(uint32_t);
+  if (ctx->replay_list.cap < need) {
+    if constexpr (sizeof(S) == 8) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      CK(cudaStreamIsCapturing(ctx->stream, &cs));
+      if (cs != cudaStreamCaptureStatusNone) return launch_persistent(ctx, ref_fn, p, b->depth, p.n);
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->replay_list.p) CK(cudaFree(ctx->replay_list.p));
+    ctx->replay_list.p = nullptr;
+    ctx->replay_list.cap = 0;
+    CK(cudaMalloc(&ctx->replay_list.p, need));
+    ctx->replay_list.cap = need;
+  }
+  CK(cudaMemsetAsync(ctx->d_replays, 0, sizeof(uint32_t), ctx->stream));
+  const bool replays = b->narrow != SQ_NARROW_AABB;
+  uint32_t* counters = nullptr;
+  int32_t rc = work_counters(ctx, replays ? 2 : 1, &counters);
+  if (rc) return rc;
+  p.replay_count = ctx->d_replays;
+  p.replay_list = static_cast<uint32_t*>(ctx->replay_list.p);
+  if ((rc = launch_persistent(ctx, fn, p, stack, p.n, counters))) return rc;
+  // A box leaf's hit is its own slab entry, so box answers are always
+  // certified and nothing is ever appended: no replay launch.
+  if (!replays) return SQ_OK;
+  // The uncertified queries again, in the reference order, unseeded.
+  QueryParamsT<S> r = p;
+  r.replay_count = nullptr;
+  r.replay_list = nullptr;
+  r.seed_bucket = nullptr;
+  r.q_list = static_cast<const uint32_t*>(ctx->replay_list.p);
+  r.q_count = ctx->d_replays;
+  return launch_persistent(ctx, ref_fn, r, b->depth, p.n, counters + 1);
+}
 
 }  // namespace sqi

@@ -33,11 +33,13 @@ template <> struct Lim<float> {
   static constexpr float eps = 1.1920928955078125e-7f;  // f32::EPSILON
   static constexpr float tri_det = 1e-8f;
   static constexpr float tri_t = 1e-6f;
+  __device__ static __forceinline__ float inf() { return __int_as_float(0x7f800000); }
 };
 template <> struct Lim<double> {
   static constexpr double eps = 2.220446049250313080847e-16;  // f64::EPSILON
   static constexpr double tri_det = 1e-8;
   static constexpr double tri_t = 1e-6;
+  __device__ static __forceinline__ double inf() { return __longlong_as_double(0x7ff0000000000000ll); }
 };
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
@@ -52,6 +54,10 @@ __device__ __forceinline__ double fmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double fdiv(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ double fsqrt(double a) { return __dsqrt_rn(a); }
 __device__ __forceinline__ double sabs(double a) { return fabs(a); }
+__device__ __forceinline__ float smin(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float smax(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double smin(double a, double b) { return fmin(a, b); }
+__device__ __forceinline__ double smax(double a, double b) { return fmax(a, b); }
 
 // Rust's f32::total_cmp / f64::total_cmp as signed keys.
 __device__ __forceinline__ int32_t total_key(float x) {
@@ -126,18 +132,17 @@ __device__ __forceinline__ bool slab(const RayPre<D, S>& r, const S* lo, const S
 // normalised with + 0. Callers use this form only for rays with no parallel
 // axis and finite origin, direction, probe and limit, against a scene whose
 // bounds are all finite; other rays take `slab`.
-template <int D>
-__device__ __forceinline__ bool slab_fast(const RayPre<D>& r, const float* lo, const float* hi, float max_toi,
-                                          float& t_enter) {
-  float tmin = 0.f, tmax = max_toi;
+template <int D, class S>
+__device__ __forceinline__ bool slab_fast(const RayPre<D, S>& r, const S* lo, const S* hi, S max_toi, S& t_enter) {
+  S tmin = S(0), tmax = max_toi;
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    const float t1 = fmul(fsub(lo[i], r.o[i]), r.inv[i]);
-    const float t2 = fmul(fsub(hi[i], r.o[i]), r.inv[i]);
-    tmin = fmaxf(tmin, fminf(t1, t2));
-    tmax = fminf(tmax, fmaxf(t1, t2));
+    const S t1 = fmul(fsub(lo[i], r.o[i]), r.inv[i]);
+    const S t2 = fmul(fsub(hi[i], r.o[i]), r.inv[i]);
+    tmin = smax(tmin, smin(t1, t2));
+    tmax = smin(tmax, smax(t1, t2));
   }
-  t_enter = fadd(tmin, 0.0f);
+  t_enter = fadd(tmin, S(0));
   return !(tmin > tmax);
 }
 
@@ -155,11 +160,10 @@ __device__ __forceinline__ bool slab_grown(const RayPre<D, S>& r, const S* lo, c
   return slab<D>(r, glo, ghi, max_toi, t_enter, axis);
 }
 
-template <int D>
-__device__ __forceinline__ bool slab_grown_fast(const RayPre<D>& r, const float* lo, const float* hi,
-                                                const float* pmin, const float* pmax, float max_toi,
-                                                float& t_enter) {
-  float glo[D], ghi[D];
+template <int D, class S>
+__device__ __forceinline__ bool slab_grown_fast(const RayPre<D, S>& r, const S* lo, const S* hi, const S* pmin,
+                                                const S* pmax, S max_toi, S& t_enter) {
+  S glo[D], ghi[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     glo[i] = fsub(lo[i], pmax[i]);

@@ -59,6 +59,7 @@ struct BlasRoot {
 };
 
 struct TlasParams {
+  static constexpr int kEntryBytes = 8;  // a stack entry: code and slab entry
   const float4* __restrict__ nodes;
   float4* insts;
   const float* root_box;

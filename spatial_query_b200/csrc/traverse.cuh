@@ -102,9 +102,11 @@ constexpr int kMaxStack = 96;  // deepest tree accepted (96 KB of stack per bloc
 // 32-byte loads (load_vec).
 __host__ __device__ constexpr int record_vec(int words) { return words <= 4 ? 1 : (words + 7) / 8 * 2; }
 
-template <int D> struct NodeLayout {
-  static constexpr int words = 4 * D + 2;  // a.lo a.hi b.lo b.hi code_a code_b
+// S: the scene's scalar; `words` counts 32-bit words.
+template <int D, class S = float> struct NodeLayout {
+  static constexpr int words = 4 * D * int(sizeof(S) / 4) + 2;  // a.lo a.hi b.lo b.hi code_a code_b
   static constexpr int vec = record_vec(words);
+  static constexpr int scalars = vec * 16 / int(sizeof(S));  // S values that hold a record
 };
 
 // Four-wide records (the binary tree with every other level folded into its
@@ -218,20 +220,24 @@ __host__ __device__ void quantize_record(const float* box, const uint32_t* codes
   }
 }
 
-template <int D, int N> struct PrimLayout {
+template <int D, int N, class S = float> struct PrimLayout {
   static constexpr int payload = (N == kNarrowAabb)     ? 2 * D
                                  : (N == kNarrowTri)    ? 9
                                  : (N == kNarrowCustom) ? SQ_CUSTOM_STRIDE + 2 * D
                                                         : D + 1;
-  static constexpr int id_word = payload;
-  static constexpr int vec = record_vec(payload + 1);
+  static constexpr int id_word = payload;  // the scalar whose (low) 32 bits are the id word
+  static constexpr int vec = record_vec((payload + 1) * int(sizeof(S) / 4));
+  static constexpr int scalars = vec * 16 / int(sizeof(S));
 };
 
 template <int K> struct QueryLayout {
   // floats per query record: rays o,d; casts o,d,probe.min,probe.max; regions lo,hi
 };
 
-struct QueryParams {
+// S: the scalar of the scene and its queries (double: the crate's f64 feature,
+// which has no seeds and no four-wide records).
+template <class S> struct QueryParamsT {
+  static constexpr int kEntryBytes = 4 + int(sizeof(S));  // a stack entry: code and slab entry
   const float4* __restrict__ nodes;
   const float4* __restrict__ wnodes;  // four-wide records (WIDE kernels)
   const float4* __restrict__ qnodes;  // quantised four-wide records (QUANT kernels; same numbering)
@@ -239,14 +245,14 @@ struct QueryParams {
   const float4* __restrict__ prims;
   const uint64_t* __restrict__ layers;
   const uint32_t* __restrict__ sub;
-  const float* __restrict__ queries;
-  const float* __restrict__ max_toi_arr;
+  const S* __restrict__ queries;
+  const S* __restrict__ max_toi_arr;
   uint32_t* counter;
   uint32_t* out_leaf;
-  float* out_toi;
+  S* out_toi;
   uint32_t* out_sub;
-  float* out_normal;
-  float* out_point;
+  S* out_normal;
+  S* out_point;
   uint32_t* out_count;
   const unsigned long long* csr_offsets;
   uint32_t* csr_leaves;
@@ -259,14 +265,14 @@ struct QueryParams {
   float window;            // relative window past the limit within which near-first still visits nodes
   unsigned long long mask;
   long long exclude;
-  const float* root_box;  // min[D], max[D] of the root (device memory: refit updates it)
+  const S* root_box;  // min[D], max[D] of the root (device memory: refit updates it)
   const int32_t* seed_bucket;  // learned guide: predicted bucket per query (seeded launches)
   const uint2* buckets;        // per bucket: node code, parent record << 1 | slot (kNoHit: the root)
   const uint32_t* bucket_sibs; // per bucket, sib_stride slots (record << 1 | slot) of its ancestors' other children
   uint32_t n_buckets;
   uint32_t sib_stride;
   const int* nonfinite;   // non-zero when some node bound is not finite (device memory)
-  float max_toi;
+  S max_toi;
   int stack;              // traversal-stack entries per thread (dynamic shared memory)
   uint32_t root_code;
   uint32_t n;
@@ -293,8 +299,9 @@ struct QueryParams {
   uint32_t* heavy_cursor;
   uint32_t heavy_cap;      // entries of heavy_store
 };
+using QueryParams = QueryParamsT<float>;
 
-__device__ __forceinline__ bool accepts(const QueryParams& p, uint32_t id) {
+template <class S> __device__ __forceinline__ bool accepts(const QueryParamsT<S>& p, uint32_t id) {
   if (!p.layers) return true;
   if (p.exclude >= 0 && (unsigned long long)p.exclude == id) return false;
   return (__ldg(p.layers + id) & p.mask) != 0ull;
@@ -331,6 +338,39 @@ template <int NV> __device__ __forceinline__ void load_vec(const float4* __restr
   }
 }
 
+template <int NV> __device__ __forceinline__ void load_vec(const float4* __restrict__ src, double* dst) {
+  if constexpr (kWideLoads && NV % 2 == 0) {
+#pragma unroll
+    for (int j = 0; j < NV / 2; ++j) {
+      double* d = dst + 4 * j;
+      asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+          : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3])
+          : "l"(src + 2 * j));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(src) + j);
+      dst[2 * j + 0] = v.x;
+      dst[2 * j + 1] = v.y;
+    }
+  }
+}
+
+// A record's 32-bit words: the id word of a primitive, the child codes of a
+// node (in f64 records, both in the scalar after the boxes).
+__device__ __forceinline__ uint32_t word_of(float x) { return __float_as_uint(x); }
+__device__ __forceinline__ uint32_t word_of(double x) { return uint32_t(__double_as_longlong(x)); }
+template <int D> __device__ __forceinline__ void node_codes(const float* rec, uint32_t& a, uint32_t& b) {
+  a = __float_as_uint(rec[4 * D]);
+  b = __float_as_uint(rec[4 * D + 1]);
+}
+template <int D> __device__ __forceinline__ void node_codes(const double* rec, uint32_t& a, uint32_t& b) {
+  const unsigned long long w = (unsigned long long)__double_as_longlong(rec[4 * D]);
+  a = uint32_t(w);
+  b = uint32_t(w >> 32);
+}
+
 // Near-first traversal visits nodes in another order than the reference, so
 // its answer is certified before it counts. The reference's limit never
 // drops below the global minimum hit h, and every box enclosing h's
@@ -350,16 +390,18 @@ template <int NV> __device__ __forceinline__ void load_vec(const float4* __restr
 __device__ __forceinline__ float near_limit(float limit, float window) {
   return __fadd_rn(limit, __fadd_rn(__fmul_rn(fabsf(limit), window), 0x1p-20f));
 }
+__device__ __forceinline__ double near_limit(double limit, float window) {
+  return __dadd_rn(limit, __dadd_rn(__dmul_rn(fabs(limit), double(window)), 0x1p-20));
+}
 
 // The slab entry of a primitive's own AABB for a ray or sweep (computed only
 // when the primitive is hit): a hit before it is a hit before every box that
 // encloses the primitive.
-template <int D, int N, bool CAST>
-__device__ __forceinline__ float prim_entry(const float* rec, const RayPre<D>& r, const float* pmin, const float* pmax,
-                                            bool fast) {
-  float lo[D], hi[D], te;
+template <int D, int N, bool CAST, class S>
+__device__ __forceinline__ S prim_entry(const S* rec, const RayPre<D, S>& r, const S* pmin, const S* pmax, bool fast) {
+  S lo[D], hi[D], te;
   int ax;
-  const float inf = __int_as_float(0x7f800000);
+  const S inf = Lim<S>::inf();
   if constexpr (N == kNarrowTri) {
     tri_aabb(rec, rec + 3, rec + 6, lo, hi);
   } else if constexpr (N == kNarrowCustom) {
@@ -392,8 +434,8 @@ __device__ __forceinline__ float prim_entry(const float* rec, const RayPre<D>& r
 }
 
 // One primitive's ray test (QueryGeometry::test_ray for the built-in providers).
-template <int D, int N>
-__device__ __forceinline__ bool narrow_ray(const float* rec, const RayPre<D>& r, float max_toi, float& t, float* n) {
+template <int D, int N, class S>
+__device__ __forceinline__ bool narrow_ray(const S* rec, const RayPre<D, S>& r, S max_toi, S& t, S* n) {
   if constexpr (N == kNarrowAabb) {
     int axis;
     if (!slab<D>(r, rec, rec + D, max_toi, t, axis)) return false;
@@ -403,7 +445,7 @@ __device__ __forceinline__ bool narrow_ray(const float* rec, const RayPre<D>& r,
     return ray_ball<D, N == kNarrowSphere>(r.o, r.d, rec, rec[D], max_toi, t, n);
   } else if constexpr (N == kNarrowCustom) {
 #ifdef SQ_RTC_CUSTOM
-    const uint32_t leaf = __float_as_uint(rec[PrimLayout<D, N>::id_word]) & ~kLeafBit;
+    const uint32_t leaf = word_of(rec[PrimLayout<D, N>::id_word]) & ~kLeafBit;
     if (!sq_narrow(rec, leaf, r.o, r.d, max_toi, &t, n)) return false;
     return !(t > max_toi);
 #else
@@ -418,9 +460,9 @@ __device__ __forceinline__ bool narrow_ray(const float* rec, const RayPre<D>& r,
 }
 
 // One primitive's swept-probe test (QueryGeometry::test_shape_cast).
-template <int D, int N>
-__device__ __forceinline__ bool narrow_cast(const float* rec, const RayPre<D>& r, const float* pmin, const float* pmax,
-                                            float max_toi, float& t, float* n) {
+template <int D, int N, class S>
+__device__ __forceinline__ bool narrow_cast(const S* rec, const RayPre<D, S>& r, const S* pmin, const S* pmax,
+                                            S max_toi, S& t, S* n) {
   if constexpr (N == kNarrowAabb) {
     int axis;
     if (!slab_grown<D>(r, rec, rec + D, pmin, pmax, max_toi, t, axis)) return false;
@@ -429,7 +471,7 @@ __device__ __forceinline__ bool narrow_cast(const float* rec, const RayPre<D>& r
   } else if constexpr (N == kNarrowSphere || N == kNarrowSphereNear) {
     return ray_ball<D, N == kNarrowSphere>(r.o, r.d, rec, fadd(rec[D], pmax[0]), max_toi, t, n);
   } else {
-    float lo[3], hi[3];
+    S lo[3], hi[3];
     tri_aabb(rec, rec + 3, rec + 6, lo, hi);
     int axis;
     if (!slab_grown<3>(r, lo, hi, pmin, pmax, max_toi, t, axis)) return false;
@@ -441,21 +483,21 @@ __device__ __forceinline__ bool narrow_cast(const float* rec, const RayPre<D>& r
 // One primitive's overlap test (QueryGeometry::test_overlap): the box itself,
 // point_to_aabb <= radius for balls (tests/shape_overlap.rs:59-72,113-115),
 // the triangle's AABB for triangles.
-template <int D, int N>
-__device__ __forceinline__ bool narrow_overlap(const float* rec, const float* qlo, const float* qhi) {
+template <int D, int N, class S>
+__device__ __forceinline__ bool narrow_overlap(const S* rec, const S* qlo, const S* qhi) {
   if constexpr (N == kNarrowAabb) {
     return box_overlap<D>(rec, rec + D, qlo, qhi);
   } else if constexpr (N == kNarrowSphere || N == kNarrowSphereNear) {
-    float d2 = 0.f;
+    S d2 = S(0);
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      float c = rec[i];
-      float v = (c < qlo[i]) ? fsub(qlo[i], c) : ((c > qhi[i]) ? fsub(c, qhi[i]) : 0.f);
+      S c = rec[i];
+      S v = (c < qlo[i]) ? fsub(qlo[i], c) : ((c > qhi[i]) ? fsub(c, qhi[i]) : S(0));
       d2 = fadd(d2, fmul(v, v));
     }
     return fsqrt(d2) <= rec[D];
   } else {
-    float lo[3], hi[3];
+    S lo[3], hi[3];
     tri_aabb(rec, rec + 3, rec + 6, lo, hi);
     return box_overlap<3>(lo, hi, qlo, qhi);
   }
@@ -464,10 +506,10 @@ __device__ __forceinline__ bool narrow_overlap(const float* rec, const float* ql
 // Sorted insertion into query q's bounded hit list (hit_ordering, stable:
 // an equal key goes after the entries already present). `count` is the full
 // number of hits so far; the first min(count, k) entries are kept.
-template <int D>
-__device__ __forceinline__ void list_put(uint32_t k, uint32_t* o_leaf, float* o_toi, uint32_t* o_sub, float* o_nrm,
-                                         uint32_t q, uint32_t& count, float t, uint32_t leaf, uint32_t subv,
-                                         const float* n) {
+template <int D, class S>
+__device__ __forceinline__ void list_put(uint32_t k, uint32_t* o_leaf, S* o_toi, uint32_t* o_sub, S* o_nrm,
+                                         uint32_t q, uint32_t& count, S t, uint32_t leaf, uint32_t subv,
+                                         const S* n) {
   uint32_t m = count < k ? count : k;
   ++count;
   if (k == 0) return;
@@ -494,31 +536,31 @@ __device__ __forceinline__ void list_put(uint32_t k, uint32_t* o_leaf, float* o_
     for (int i = 0; i < D; ++i) o_nrm[(base + j) * D + i] = n[i];
 }
 
-template <int D>
-__device__ __forceinline__ void list_insert(const QueryParams& p, uint32_t q, uint32_t& count, float t, uint32_t leaf,
-                                            const float* n) {
+template <int D, class S>
+__device__ __forceinline__ void list_insert(const QueryParamsT<S>& p, uint32_t q, uint32_t& count, S t, uint32_t leaf,
+                                            const S* n) {
   list_put<D>(p.k, p.out_leaf, p.out_toi, p.out_sub, p.out_normal, q, count, t, leaf,
               p.sub ? __ldg(p.sub + leaf) : kNoHit, n);
 }
 
 // Per-lane traversal state of one query.
-template <int D, int K> struct Lane {
-  RayPre<D> r;
-  float pmin[D], pmax[D];
-  float limit;       // nodes whose entry lies past this are pruned (near-first: the best hit plus the window)
+template <int D, int K, class S> struct Lane {
+  RayPre<D, S> r;
+  S pmin[D], pmax[D];
+  S limit;       // nodes whose entry lies past this are pruned (near-first: the best hit plus the window)
   uint32_t best_pos; // primitive position of the best hit (its certification and normal)
   uint32_t q;
   uint32_t code;
-  float code_t;      // entry of the node in code (postponed-leaf walks re-check it after a leaf)
+  S code_t;      // entry of the node in code (postponed-leaf walks re-check it after a leaf)
   uint32_t top_code; // postponed-leaf walks: the stack's top entry, held in registers
-  float top_t;
+  S top_t;
   bool has_top;
   int sp;
   bool fast;
   uint32_t best_leaf;
-  float best_t;
-  float second_t;    // near-first: the nearest of the query's other hits
-  float best_n[D];   // consumer narrow phases only
+  S best_t;
+  S second_t;    // near-first: the nearest of the query's other hits
+  S best_n[D];   // consumer narrow phases only
   uint32_t count;
   unsigned long long csr_base;
   uint32_t v_nodes, v_nar, v_hit;
@@ -529,9 +571,11 @@ template <int D, int K> struct Lane {
 // spill). At D = 3 and 1,048,576 terrain rays, 7 / 8 / 9 / 10 blocks measured
 // 512 / 464 / 441 / 483 us (nine: 56 registers, no spills; ten: 48 registers,
 // 32 bytes spilled). Longer rays and records (D = 4 and 6, casts, four-wide
-// records) need more registers each.
-__host__ __device__ constexpr int resident_blocks(int D, int kind, bool stats, bool wide) {
-  if (stats) return 1;
+// records) need more registers each. Doubles are left to the compiler (200,000
+// boxes, 100,001 host rays: 708 us at the natural 88 registers, 691 / 699 / 709
+// at 4 / 5 / 6 blocks).
+__host__ __device__ constexpr int resident_blocks(int D, int kind, bool stats, bool wide, bool f64) {
+  if (stats || f64) return 1;
   if (wide) return D <= 3 ? 8 : (D == 4 ? 6 : 5);
   if (D <= 3 || kind == kOverlap) return 9;
   if (kind == kCastNearest || kind == kCastAll) return D == 4 ? 7 : 5;
@@ -571,30 +615,29 @@ __host__ __device__ constexpr int resident_blocks(int D, int kind, bool stats, b
 // postponed leaves with the stack's top entry held in registers; 2 = child
 // order by warp vote.
 template <int D, int N, int K, bool REF, bool STATS, bool SEED = false, bool WIDE = false, bool QUANT = false,
-          int WALK = 0>
-__global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) query_kernel(const QueryParams p) {
+          int WALK = 0, class S = float>
+__global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE, sizeof(S) == 8)) query_kernel(const QueryParamsT<S> p) {
   static_assert(!WIDE || (K == kRayNearest && !REF && !STATS && !SEED), "four-wide walks serve near-first rays only");
   static_assert(!QUANT || WIDE, "quantised records are a four-wide layout");
   constexpr bool kNearest = (K == kRayNearest || K == kCastNearest);
   constexpr bool kCast = (K == kCastNearest || K == kCastAll);
   constexpr bool kList = (K == kRayAll || K == kCastAll);
   constexpr int QW = kCast ? 4 * D : 2 * D;
-  using PL = PrimLayout<D, N>;
-  using NL = NodeLayout<D>;
+  using PL = PrimLayout<D, N, S>;
+  using NL = NodeLayout<D, S>;
   using WL = WideLayout<D>;
   constexpr uint32_t FULL = 0xffffffffu;
 
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const int S = p.stack;
-  uint32_t* s_code = smem;
-  float* s_t = reinterpret_cast<float*>(smem + S * kThreads);
+  S* s_t = reinterpret_cast<S*>(smem);
+  uint32_t* s_code = reinterpret_cast<uint32_t*>(s_t + p.stack * kThreads);
   const uint32_t lt_mask = (1u << lane) - 1u;
   const bool scene_finite = p.nonfinite ? (*p.nonfinite == 0) : true;
 
   unsigned long long c_vis = 0, c_nar = 0, c_hit = 0;
-  Lane<D, K> L;
+  Lane<D, K, S> L;
   const uint32_t n_queries = p.q_count ? *p.q_count : p.n;
 
   constexpr bool DETECT = kNearest && !REF;
@@ -606,14 +649,14 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
   // Idle lanes help where the answer does not depend on the order of the
   // visits and no counter reports them.
   constexpr bool HELP = DETECT && !STATS && !SPEC;
-  const float kInf = __int_as_float(0x7f800000);
+  const S kInf = Lim<S>::inf();
 
   // Box test of one child (or the root) against the lane's query: the slab
   // without the limit, then the entry against the limit (the same verdict as
   // the reference's slab clipped to the limit, aabb.rs:118-148).
-  auto test_box = [&](const float* lo, const float* hi, float& te) -> bool {
+  auto test_box = [&](const S* lo, const S* hi, S& te) -> bool {
     if constexpr (K == kOverlap) {
-      te = 0.f;
+      te = S(0);
       return box_overlap<D>(lo, hi, L.r.o, L.r.d);  // region lo / hi sit in o / d
     } else {
       bool geo;
@@ -642,7 +685,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
     while (L.sp > lo) {
       --L.sp;
       L.code = s_code[L.sp * kThreads + tid];
-      const float t = s_t[L.sp * kThreads + tid];
+      const S t = s_t[L.sp * kThreads + tid];
       L.code_t = t;
       if (!kNearest || t <= L.limit) return true;
     }
@@ -651,17 +694,17 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
 
   auto finish = [&]() {
     const uint32_t q = L.q;
-    float nrm[D];
+    S nrm[D];
     if constexpr (kNearest) {
 #pragma unroll
-      for (int i = 0; i < D; ++i) nrm[i] = N == kNarrowCustom ? L.best_n[i] : 0.f;
+      for (int i = 0; i < D; ++i) nrm[i] = N == kNarrowCustom ? L.best_n[i] : S(0);
       if (L.best_leaf != kNoHit && ((DETECT && N != kNarrowAabb) || (N != kNarrowCustom && p.out_normal))) {
-        float rec[PL::vec * 4];
+        S rec[PL::scalars];
         load_vec<PL::vec>(p.prims + size_t(L.best_pos) * PL::vec, rec);
         // Certify the answer: not before its own primitive's AABB entry.
         if constexpr (DETECT && N != kNarrowAabb) {
-          const float te = prim_entry<D, N, kCast>(rec, L.r, L.pmin, L.pmax, L.fast);
-          const float mt = p.max_toi_arr ? p.max_toi_arr[q] : p.max_toi;
+          const S te = prim_entry<D, N, kCast>(rec, L.r, L.pmin, L.pmax, L.fast);
+          const S mt = p.max_toi_arr ? p.max_toi_arr[q] : p.max_toi;
           if (L.best_t < te && !(te <= mt && te <= near_limit(L.best_t, p.window) && te <= L.second_t))
             p.replay_list[atomicAdd(p.replay_count, 1u)] = q;
         }
@@ -669,7 +712,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
         // primitive bounded by the hit itself.
         if constexpr (N != kNarrowCustom) {
           if (p.out_normal) {
-            float t;
+            S t;
             if constexpr (kCast) narrow_cast<D, N>(rec, L.r, L.pmin, L.pmax, L.best_t, t, nrm);
             else if constexpr (N == kNarrowTri) tri_normal(rec, rec + 3, rec + 6, nrm);
             else narrow_ray<D, N>(rec, L.r, L.best_t, t, nrm);
@@ -686,12 +729,12 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
         for (int i = 0; i < D; ++i) p.out_normal[size_t(q) * D + i] = nrm[i];
       }
       if (p.out_point) {
-        float pt[D];
+        S pt[D];
         if (L.best_leaf != kNoHit) {
           ray_at<D>(L.r.o, L.r.d, L.best_t, pt);
         } else {
 #pragma unroll
-          for (int i = 0; i < D; ++i) pt[i] = 0.f;
+          for (int i = 0; i < D; ++i) pt[i] = S(0);
         }
 #pragma unroll
         for (int i = 0; i < D; ++i) p.out_point[size_t(q) * D + i] = pt[i];
@@ -726,7 +769,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
   // Loads query q and tests the root. False when the query is already done.
   auto start = [&](uint32_t q) -> bool {
     L.q = q;
-    const float* src = p.queries + size_t(q) * QW;
+    const S* src = p.queries + size_t(q) * QW;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
       L.r.o[i] = src[i];
@@ -750,11 +793,11 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
       L.fast = false;
     }
     L.best_leaf = kNoHit;
-    L.best_t = 0.f;
+    L.best_t = S(0);
     L.second_t = kInf;
     if constexpr (N == kNarrowCustom) {
 #pragma unroll
-      for (int i = 0; i < D; ++i) L.best_n[i] = 0.f;
+      for (int i = 0; i < D; ++i) L.best_n[i] = S(0);
     }
     L.count = 0;
     L.csr_base = 0;
@@ -796,13 +839,13 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
     L.sp = 0;
     L.has_top = false;
     L.code = WIDE ? p.wroot : p.root_code;
-    float lo[D], hi[D];
+    S lo[D], hi[D];
 #pragma unroll
     for (int i = 0; i < D; ++i) {
       lo[i] = p.root_box[i];
       hi[i] = p.root_box[D + i];
     }
-    float te;
+    S te;
     const bool hit_root = test_box(lo, hi, te);
     L.code_t = te;
     if constexpr (SEED) {
@@ -810,10 +853,10 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
       if (hit_root && bk >= 0 && uint32_t(bk) < p.n_buckets) {
         const uint2 e = __ldg(p.buckets + bk);
         if (e.x != p.root_code) {
-          const float* box = (e.y == kNoHit) ? p.root_box
+          const S* box = (e.y == kNoHit) ? p.root_box
                                              : reinterpret_cast<const float*>(p.nodes + size_t(e.y >> 1) * NL::vec) +
                                                    (e.y & 1u) * 2 * D;
-          float blo[D], bhi[D], tb;
+          S blo[D], bhi[D], tb;
 #pragma unroll
           for (int i = 0; i < D; ++i) {
             blo[i] = box[i];
@@ -830,17 +873,17 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
             for (uint32_t i = 0; i < p.sib_stride; ++i) {
               const uint32_t sl = __ldg(sibs + i);
               if (sl == kNoHit) break;
-              float rec[NL::vec * 4];
+              S rec[NL::scalars];
               load_vec<NL::vec>(p.nodes + size_t(sl >> 1) * NL::vec, rec);
               const bool second = (sl & 1u) != 0u;
-              float slo[D], shi[D];
+              S slo[D], shi[D];
 #pragma unroll
               for (int k = 0; k < D; ++k) {
                 slo[k] = second ? rec[2 * D + k] : rec[k];
                 shi[k] = second ? rec[3 * D + k] : rec[D + k];
               }
               const uint32_t sc = __float_as_uint(second ? rec[4 * D + 1] : rec[4 * D]);
-              float ts;
+              S ts;
               if (STATS) L.v_nodes += 1;
               if (test_box(slo, shi, ts)) {
                 s_code[L.sp * kThreads + tid] = sc;
@@ -858,11 +901,11 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
   };
 
   // A hit of the lane's query: kept when it is before the best one.
-  auto take_hit = [&](float t, uint32_t id, uint32_t pos) -> bool {
+  auto take_hit = [&](S t, uint32_t id, uint32_t pos) -> bool {
     const bool first = L.best_leaf == kNoHit || hit_before(t, id, L.best_t, L.best_leaf);
     if constexpr (DETECT && N != kNarrowAabb) {
       // The nearest of the other hits; a NaN marks the query uncertified.
-      const float other = first ? (L.best_leaf == kNoHit ? kInf : L.best_t) : t;
+      const S other = first ? (L.best_leaf == kNoHit ? kInf : L.best_t) : t;
       if (!(other >= L.second_t)) L.second_t = other == other ? other : -kInf;
     }
     if (first) {
@@ -875,9 +918,9 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
   };
 
   // Tests the primitive record at position pos. True: the last of its leaf.
-  auto prim = [&](const float* rec, uint32_t pos) -> bool {
+  auto prim = [&](const S* rec, uint32_t pos) -> bool {
     {
-      const uint32_t idw = __float_as_uint(rec[PL::id_word]);
+      const uint32_t idw = word_of(rec[PL::id_word]);
       const uint32_t id = idw & ~kLeafBit;
       if (accepts(p, id)) {
         if constexpr (K == kOverlap) {
@@ -900,7 +943,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
           }
         } else {
           if (STATS) L.v_nar += 1;
-          float t, nrm[D];
+          S t, nrm[D];
           if constexpr (K == kRayNearest || K == kCastNearest) {
             bool h;
             if constexpr (K == kRayNearest) h = narrow_ray<D, N>(rec, L.r, L.limit, t, nrm);
@@ -918,19 +961,19 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
             if constexpr (N == kNarrowSphere) {
               if (p.crossings) {
                 // Both roots of the unbounded ray (tests/crossings.rs:505-521).
-                float oc[D];
+                S oc[D];
 #pragma unroll
                 for (int i = 0; i < D; ++i) oc[i] = fsub(L.r.o[i], rec[i]);
-                const float b = pdot<D>(oc, L.r.d);
-                const float disc = fsub(fmul(b, b), fsub(pdot<D>(oc, oc), fmul(rec[D], rec[D])));
-                if (!(disc < 0.f)) {
-                  const float sq = fsqrt(disc);
-                  const float roots[2] = {fsub(-b, sq), fadd(-b, sq)};
+                const S b = pdot<D>(oc, L.r.d);
+                const S disc = fsub(fmul(b, b), fsub(pdot<D>(oc, oc), fmul(rec[D], rec[D])));
+                if (!(disc < S(0))) {
+                  const S sq = fsqrt(disc);
+                  const S roots[2] = {fsub(-b, sq), fadd(-b, sq)};
 #pragma unroll
                   for (int j = 0; j < 2; ++j) {
-                    const float tt = roots[j];
-                    if (tt >= 0.f && tt <= L.limit) {
-                      float pt[D];
+                    const S tt = roots[j];
+                    if (tt >= S(0) && tt <= L.limit) {
+                      S pt[D];
                       ray_at<D>(L.r.o, L.r.d, tt, pt);
 #pragma unroll
                       for (int i = 0; i < D; ++i) nrm[i] = fsub(pt[i], rec[i]);
@@ -950,7 +993,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
               if constexpr (N == kNarrowCustom) {
                 if (p.crossings) {
                   // Every crossing the consumer emits is listed, as bvh.rs:309-315 pushes them.
-                  auto emit = [&](float tt, const float* nn) {
+                  auto emit = [&](S tt, const S* nn) {
                     if (STATS) L.v_hit += 1;
                     list_insert<D>(p, L.q, L.count, tt, id, nn);
                   };
@@ -975,7 +1018,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
   // Tests the primitives of a leaf.
   auto leaf = [&](uint32_t code) {
     for (uint32_t pos = code & ~kLeafBit;; ++pos) {
-      float rec[PL::vec * 4];
+      S rec[PL::scalars];
       load_vec<PL::vec>(p.prims + size_t(pos) * PL::vec, rec);
       if (prim(rec, pos)) break;
     }
@@ -1000,14 +1043,14 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             c4[k] = qw[QL::o_code + k];
-            float lo[D], hi[D];
+            S lo[D], hi[D];
 #pragma unroll
             for (int i = 0; i < D; ++i) {
               const float step = q_step(q_byte(qw + QL::o_exp, i));
               lo[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + i), step);
               hi[i] = q_decode(qf[i], q_byte(qw + QL::o_q, 2 * D * k + D + i), step);
             }
-            float te = kInf;
+            S te = kInf;
             if (c4[k] == kNoHit || !test_box(lo, hi, te)) {
               c4[k] = kNoHit;
               te = kInf;
@@ -1018,12 +1061,12 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
         }
       }
       if (exact) {
-        float rec[WL::vec * 4];
+        S rec[WL::vec * 4];
         load_vec<WL::vec>(p.wnodes + size_t(L.code) * WL::vec, rec);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           c4[i] = __float_as_uint(rec[8 * D + i]);
-          float te = kInf;
+          S te = kInf;
           if (c4[i] == kNoHit || !test_box(rec + 2 * D * i, rec + 2 * D * i + D, te)) {
             c4[i] = kNoHit;
             te = kInf;
@@ -1062,11 +1105,11 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
       }
       return false;
     }
-    float rec[NL::vec * 4];
+    S rec[NL::scalars];
     load_vec<NL::vec>(p.nodes + size_t(L.code) * NL::vec, rec);
-    const uint32_t ca = __float_as_uint(rec[4 * D]);
-    const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
-    float ta, tb;
+    uint32_t ca, cb;
+    node_codes<D>(rec, ca, cb);
+    S ta, tb;
     const bool pa = test_box(rec, rec + D, ta);
     const bool pb = test_box(rec + 2 * D, rec + 3 * D, tb);
     if (STATS) L.v_nodes += 2;
@@ -1183,17 +1226,17 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
                 if (!pop(0)) empty = true;
               }
             } else {
-              float rec[NL::vec * 4];
+              S rec[NL::scalars];
               load_vec<NL::vec>(p.nodes + size_t(L.code) * NL::vec, rec);
               const uint32_t ca = __float_as_uint(rec[4 * D]);
               const uint32_t cb = __float_as_uint(rec[4 * D + 1]);
-              float ta, tb;
+              S ta, tb;
               const bool pa = test_box(rec, rec + D, ta);
               const bool pb = test_box(rec + 2 * D, rec + 3 * D, tb);
               if (pa && pb) {
                 const bool a_first = (SEED && p.far_first) ? false : (ta <= tb);
                 const uint32_t far_code = a_first ? cb : ca;
-                const float far_t = a_first ? tb : ta;
+                const S far_t = a_first ? tb : ta;
                 if constexpr (kRegTop) {
                   if (L.has_top) {  // the register entry spills below the new one
                     s_code[L.sp * kThreads + tid] = L.top_code;
@@ -1258,11 +1301,11 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
           const int h = __ffs(found) - 1;
           found &= found - 1u;
           const int to = __shfl_sync(FULL, owner, h);
-          const float t = __shfl_sync(FULL, L.best_t, h);
-          const float t2 = __shfl_sync(FULL, L.second_t, h);
+          const S t = __shfl_sync(FULL, L.best_t, h);
+          const S t2 = __shfl_sync(FULL, L.second_t, h);
           const uint32_t id = __shfl_sync(FULL, L.best_leaf, h);
           const uint32_t pos = __shfl_sync(FULL, L.best_pos, h);
-          float n[D];
+          S n[D];
           if constexpr (N == kNarrowCustom) {
 #pragma unroll
             for (int i = 0; i < D; ++i) n[i] = __shfl_sync(FULL, L.best_n[i], h);
@@ -1280,7 +1323,7 @@ __global__ void __launch_bounds__(kThreads, resident_blocks(D, K, STATS, WIDE)) 
             L.second_t = kInf;
           }
         }
-        L.limit = fminf(L.limit, __shfl_sync(FULL, L.limit, owner));
+        L.limit = smin(L.limit, __shfl_sync(FULL, L.limit, owner));
         // A query that no lane walks any more is answered.
         if (!live && owner != lane) owner = lane;  // a helper that has finished is free
         uint32_t walked = 0u;                       // owners of the walking lanes
@@ -1690,6 +1733,20 @@ struct KernelSet {
 };
 
 #ifndef __CUDACC_RTC__  // host code: not part of a run-time compiled unit
+// The kernels of an f64 scene (the others stay null).
+template <int D, int N> KernelSet make_kernel_set64() {
+  KernelSet s{};
+  s.ray_nearest[0][0] = (const void*)query_kernel<D, N, kRayNearest, false, false, false, false, false, 0, double>;
+  s.ray_nearest[1][0] = (const void*)query_kernel<D, N, kRayNearest, true, false, false, false, false, 0, double>;
+  s.ray_nearest[1][1] = (const void*)query_kernel<D, N, kRayNearest, true, true, false, false, false, 0, double>;
+  s.ray_all[0] = (const void*)query_kernel<D, N, kRayAll, true, false, false, false, false, 0, double>;
+  s.cast_nearest[0] = (const void*)query_kernel<D, N, kCastNearest, false, false, false, false, false, 0, double>;
+  s.cast_nearest[1] = (const void*)query_kernel<D, N, kCastNearest, true, false, false, false, false, 0, double>;
+  s.cast_all = (const void*)query_kernel<D, N, kCastAll, true, false, false, false, false, 0, double>;
+  s.overlap = (const void*)query_kernel<D, N, kOverlap, true, false, false, false, false, 0, double>;
+  return s;
+}
+
 template <int D, int N> KernelSet make_kernel_set() {
   KernelSet s;
   s.ray_nearest[0][0] = (const void*)query_kernel<D, N, kRayNearest, false, false>;

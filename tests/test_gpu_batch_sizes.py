@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+import spatial_query_b200 as sq
 from gpu_util import bits, ctx, pair
 from spatial_query_b200 import scenes
 
@@ -78,3 +79,49 @@ def test_hits_before_their_own_boxes(window):
         same_prefix(o.nearest(rays, limits), g.raycast_nearest(rays, limits), n)
     finally:
         ctx().set_replay_window(2.0 ** -16)
+
+
+def scene64(kind, dim, prims):
+    geom = sq.Geometry(kind, dim, prims)
+    return O.Scene(kind, dim, prims, prec=64), sq.DeviceBvh64(ctx(), sq.HostBvh.build_f64(dim, geom.world_aabbs_f64()),
+                                                             geom)
+
+
+def same64(ref, h, n):
+    assert np.array_equal(ref.leaf[:n], h.leaf), n
+    hit = ref.leaf[:n] != O.NO_HIT
+    assert np.array_equal(ref.toi[:n][hit].view(np.uint64), h.toi[hit].view(np.uint64)), n
+
+
+@pytest.mark.parametrize("kind,dim", [("boxes", 2), ("boxes", 6), ("balls", 3), ("tris", 3)])
+def test_batch_sizes_f64(kind, dim):
+    o, g = scene64(kind, dim, leaves(kind, dim, 3000, 5))
+    rays = rays_for(kind, dim, 100_001, 9).astype(np.float64)
+    ref = o.nearest(rays, 700.0)
+    for n in (1, 33, 5000, 100_001):  # thinly dealt, a share per warp, dynamic refill
+        same64(ref, g.raycast_nearest(rays[:n], 700.0), n)
+    half = np.full((5000, dim), 0.75)
+    casts = np.concatenate([rays[:5000], -half, half], axis=1)
+    same64(o.shapecast_nearest(casts, 300.0), g.shapecast_nearest(casts, 300.0), 5000)
+
+
+def test_f64_call_captured_on_a_fresh_context():
+    """A first f64 call inside a capture (no replay list yet) is answered."""
+    import torch
+    fresh = sq.Context(0)
+    prims = leaves("balls", 3, 3000, 5)
+    geom = sq.Geometry("balls", 3, prims)
+    g = sq.DeviceBvh64(fresh, sq.HostBvh.build_f64(3, geom.world_aabbs_f64()), geom)
+    rays = rays_for("balls", 3, 3001, 4).astype(np.float64)
+    d = torch.from_numpy(rays).cuda()
+    leaf, toi = torch.full((3001,), 7, dtype=torch.int32, device="cuda"), torch.zeros(3001, dtype=torch.float64,
+                                                                                       device="cuda")
+    torch.cuda.synchronize()
+    fresh.graph_begin()
+    fresh.check(sq.lib().sq_raycast_nearest_f64_d(fresh.h, g.h, d.data_ptr(), 3001, 700.0, None, None, leaf.data_ptr(),
+                                                  toi.data_ptr(), None, None), "nearest")
+    graph = fresh.graph_end()
+    graph.launch()
+    fresh.synchronize()
+    ref = O.Scene("balls", 3, prims, prec=64).nearest(rays, 700.0)
+    same64(ref, sq.Hits(leaf.cpu().numpy().view(np.uint32), toi.cpu().numpy()), 3001)
