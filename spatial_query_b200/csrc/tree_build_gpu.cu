@@ -9,14 +9,23 @@
 //
 // How: the recursion runs a level at a time. For every segment of a level
 // (a node's range of the primitive order) the node's box and its centroid
-// box are reduced (one warp per segment on the wide levels; many blocks per
-// segment with order-preserving integer atomics on the top levels, whose
-// few segments are long), leaf or split is decided, and each primitive of a
-// split segment gets the sort key (segment start << 32 | its split-axis key);
-// every other position keeps (position << 32). One stable radix sort of the
-// level on those keys then orders every split segment in place, which is the
-// per-node stable sort of the crate (ties keep the order the parent's sort
-// left), and leaves every other position where it is. Nodes are numbered in
+// box are reduced, leaf or split is decided, and a split segment is sorted.
+//
+// Top levels (segments longer than kBlockSort): many blocks per segment
+// reduce with order-preserving integer atomics, each primitive of a split
+// segment gets the sort key (segment start >> shift) << 32 | its split-axis
+// key, every other position (position >> shift) << 32, and one stable radix
+// sort of the level orders every split segment in place: the per-node stable
+// sort of the crate (ties keep the order the parent's sort left). shift is the
+// largest that keeps the level's segment starts apart (segments are at least
+// n >> L long, and 2^shift at most that), so level L's keys have 33 + L bits
+// instead of 32 + log2 n; a position outside the split segments that shares its
+// high word with one lies before it and sorts before it (its low word is 0).
+//
+// The levels below: a segment fits a block's shared memory, so one block (or,
+// below 33 primitives, a few lanes) reduces it, decides, and sorts it there by
+// (key, position), with no keys in memory and no radix passes. Terrain of
+// 1,048,576 triangles: 5,064 -> 2,705 us. Nodes are numbered in
 // level order as they are made; preorder numbers follow from subtree sizes
 // (bottom-up, a level at a time) and left-subtree offsets (top-down).
 //
@@ -78,14 +87,17 @@ struct LevelParams {
   const uint32_t* idx;   // the current primitive order
   const Seg* cur;
   const uint32_t* m;     // segments of this level (device memory)
+  uint32_t* order;       // small segments: the primitive order, sorted in place (same array as idx)
   Seg* next;             // the next level's segments (appended)
   uint32_t* counters;    // [0] next segments, [1] nodes made, [2] split segments
   LNode* nodes;          // by level-order id
   float* bounds;         // by level-order id: min[D], max[D]
-  unsigned long long* sort_keys;  // per position: (segment start << 32) | split-axis key, or (position << 32)
+  unsigned long long* sort_keys;  // per position: (segment start >> shift) << 32 | split-axis key, or (position >> shift) << 32
   uint32_t* red;         // top levels: per segment 4 x kMaxDim ordered bounds (box lo, hi, centroid lo, hi)
   int* axis;             // top levels: per segment the split axis, -1 for a leaf
   uint32_t chunk;        // top levels: positions per block
+  uint32_t chunks;       // top levels: blocks per segment
+  uint32_t shift;        // top levels: positions >> shift tell the level's segments apart
 };
 
 // f32 <-> an unsigned key with the same order (total_ukey), for min / max
@@ -141,9 +153,9 @@ __global__ void advance_kernel(uint32_t* counters, uint32_t* level_info, uint32_
 }
 
 // Every position keeps its place unless a split segment claims it.
-__global__ void place_keys_kernel(unsigned long long* sort_keys, uint32_t n) {
+__global__ void place_keys_kernel(unsigned long long* sort_keys, uint32_t n, uint32_t shift) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    sort_keys[i] = (unsigned long long)i << 32;
+    sort_keys[i] = (unsigned long long)(i >> shift) << 32;
 }
 
 // Top levels: empty per-segment bounds (+inf for the minima, -inf for the maxima).
@@ -154,13 +166,13 @@ __global__ void red_init_kernel(uint32_t* red, uint32_t m) {
   red[i] = (part == 0 || part == 2) ? total_ukey(INFINITY) : total_ukey(-INFINITY);
 }
 
-// Top levels: block (c, g) reduces positions [s + c * chunk, s + (c + 1) * chunk)
-// of segment g and folds its result into the segment's bounds.
+// Top levels: block g * chunks + c reduces positions [s + c * chunk, s + (c + 1)
+// * chunk) of segment g and folds its result into the segment's bounds.
 __global__ void __launch_bounds__(256) red_kernel(const LevelParams p) {
-  const uint32_t g = blockIdx.y;
+  const uint32_t g = blockIdx.x / p.chunks;
   if (g >= *p.m) return;  // the grid covers the level's bound
   const Seg sg = p.cur[g];
-  const uint64_t b0 = uint64_t(sg.s) + uint64_t(blockIdx.x) * p.chunk;
+  const uint64_t b0 = uint64_t(sg.s) + uint64_t(blockIdx.x % p.chunks) * p.chunk;
   if (b0 >= sg.e) return;  // uniform per block
   const uint32_t b1 = uint32_t(std::min<uint64_t>(sg.e, b0 + p.chunk));
   const int D = p.D;
@@ -223,51 +235,39 @@ __global__ void decide_kernel(const LevelParams p) {
 
 // Top levels: the sort keys of the split segments' positions, chunked like red_kernel.
 __global__ void split_keys_kernel(const LevelParams p) {
-  const uint32_t g = blockIdx.y;
+  const uint32_t g = blockIdx.x / p.chunks;
   if (g >= *p.m) return;
   const int axis = p.axis[g];
   if (axis < 0) return;
   const Seg sg = p.cur[g];
-  const uint64_t b0 = uint64_t(sg.s) + uint64_t(blockIdx.x) * p.chunk;
+  const uint64_t b0 = uint64_t(sg.s) + uint64_t(blockIdx.x % p.chunks) * p.chunk;
   if (b0 >= sg.e) return;
   const uint32_t b1 = uint32_t(std::min<uint64_t>(sg.e, b0 + p.chunk));
   const uint32_t* key = p.keys + size_t(axis) * p.n;
   for (uint32_t pos = uint32_t(b0) + threadIdx.x; pos < b1; pos += blockDim.x)
-    p.sort_keys[pos] = ((unsigned long long)sg.s << 32) | key[p.idx[pos]];
+    p.sort_keys[pos] = ((unsigned long long)(sg.s >> p.shift) << 32) | key[p.idx[pos]];
 }
 
-// Wide levels: one warp per segment.
-template <int TPS>
-__global__ void __launch_bounds__(256) level_kernel(const LevelParams p) {
-  static_assert(TPS == 32, "one warp per segment");
-  const uint32_t groups = blockDim.x / TPS;
-  const uint32_t g = blockIdx.x * groups + threadIdx.x / TPS;
-  const uint32_t lane = threadIdx.x % TPS;
-  if (g >= *p.m) return;  // uniform per warp
-  const int D = p.D;
-  const Seg sg = p.cur[g];
-  float lo[kMaxDim], hi[kMaxDim], clo[kMaxDim], chi[kMaxDim];
+// Folds primitive id's box and centroid into a segment's reduction.
+__device__ __forceinline__ void fold_box(const LevelParams& p, uint32_t id, float* lo, float* hi, float* clo, float* chi) {
+  const float* b = p.aabbs + size_t(id) * 2 * p.D;
 #pragma unroll
   for (int k = 0; k < kMaxDim; ++k) {
-    lo[k] = clo[k] = INFINITY;
-    hi[k] = chi[k] = -INFINITY;
-  }
-  for (uint32_t pos = sg.s + lane; pos < sg.e; pos += TPS) {
-    const float* b = p.aabbs + size_t(p.idx[pos]) * 2 * D;
-#pragma unroll
-    for (int k = 0; k < kMaxDim; ++k) {
-      if (k < D) {
-        lo[k] = fminf(lo[k], b[k]);
-        hi[k] = fmaxf(hi[k], b[D + k]);
-        const float c = centre(b, D, k);
-        clo[k] = fminf(clo[k], c);
-        chi[k] = fmaxf(chi[k], c);
-      }
+    if (k < p.D) {
+      lo[k] = fminf(lo[k], b[k]);
+      hi[k] = fmaxf(hi[k], b[p.D + k]);
+      const float c = centre(b, p.D, k);
+      clo[k] = fminf(clo[k], c);
+      chi[k] = fmaxf(chi[k], c);
     }
   }
-  // Group reduction (min / max are exact in any order).
+}
+
+// The reduction over groups of TPS lanes (min / max are exact in any order).
+template <int TPS>
+__device__ __forceinline__ void reduce_lanes(int D, float* lo, float* hi, float* clo, float* chi) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = TPS / 2; o > 0; o >>= 1) {
 #pragma unroll
     for (int k = 0; k < kMaxDim; ++k) {
       if (k < D) {
@@ -278,14 +278,118 @@ __global__ void __launch_bounds__(256) level_kernel(const LevelParams p) {
       }
     }
   }
-  // Leaf or split, decided by the warp's first lane.
-  int axis = -1;
-  if (lane == 0) axis = decide(p, sg, lo, hi, clo, chi);
-  axis = __shfl_sync(0xffffffffu, axis, 0);
-  if (axis < 0) return;
+}
+
+__device__ __forceinline__ void empty_box(float* lo, float* hi, float* clo, float* chi) {
+#pragma unroll
+  for (int k = 0; k < kMaxDim; ++k) {
+    lo[k] = clo[k] = INFINITY;
+    hi[k] = chi[k] = -INFINITY;
+  }
+}
+
+// Segments of up to kBlockSort primitives, one block each: reduced, decided
+// and sorted in shared memory (bitonic over (key, position) words, unique, so
+// the order is the stable sort's). Dynamic shared memory: `padded` sort words
+// (a power of two, no less than the level's longest segment), then as many ids.
+constexpr uint32_t kBlockSort = 2048;
+__global__ void __launch_bounds__(256) level_block_kernel(const LevelParams p, uint32_t padded) {
+  extern __shared__ unsigned long long s_word[];
+  __shared__ float s_red[8][4 * kMaxDim];
+  __shared__ int s_axis;
+  const uint32_t g = blockIdx.x;
+  if (g >= *p.m) return;  // uniform per block
+  const int D = p.D;
+  const Seg sg = p.cur[g];
+  const uint32_t count = sg.e - sg.s;
+  uint32_t* s_id = reinterpret_cast<uint32_t*>(s_word + padded);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float lo[kMaxDim], hi[kMaxDim], clo[kMaxDim], chi[kMaxDim];
+  empty_box(lo, hi, clo, chi);
+  for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
+    const uint32_t id = p.order[sg.s + i];
+    s_id[i] = id;
+    fold_box(p, id, lo, hi, clo, chi);
+  }
+  reduce_lanes<32>(D, lo, hi, clo, chi);
+  if (lane == 0) {
+    for (int k = 0; k < D; ++k) {
+      s_red[warp][k] = lo[k];
+      s_red[warp][kMaxDim + k] = hi[k];
+      s_red[warp][2 * kMaxDim + k] = clo[k];
+      s_red[warp][3 * kMaxDim + k] = chi[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t w = 1; w < blockDim.x / 32; ++w) {
+      for (int k = 0; k < D; ++k) {
+        lo[k] = fminf(lo[k], s_red[w][k]);
+        hi[k] = fmaxf(hi[k], s_red[w][kMaxDim + k]);
+        clo[k] = fminf(clo[k], s_red[w][2 * kMaxDim + k]);
+        chi[k] = fmaxf(chi[k], s_red[w][3 * kMaxDim + k]);
+      }
+    }
+    s_axis = decide(p, sg, lo, hi, clo, chi);
+  }
+  __syncthreads();
+  const int axis = s_axis;
+  if (axis < 0) return;  // uniform per block
   const uint32_t* key = p.keys + size_t(axis) * p.n;
-  for (uint32_t pos = sg.s + lane; pos < sg.e; pos += TPS)
-    p.sort_keys[pos] = ((unsigned long long)sg.s << 32) | key[p.idx[pos]];
+  uint32_t m = 32;
+  while (m < count) m <<= 1;  // sorted width: at most `padded`
+  for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
+    s_word[i] = i < count ? ((unsigned long long)key[s_id[i]] << 32) | i : ~0ull;
+  __syncthreads();
+  for (uint32_t k = 2; k <= m; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      for (uint32_t t = threadIdx.x; t < m / 2; t += blockDim.x) {
+        const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;
+        const unsigned long long x = s_word[a], y = s_word[b];
+        if ((x > y) == ((a & k) == 0)) {
+          s_word[a] = y;
+          s_word[b] = x;
+        }
+      }
+      // Pairs of one warp's words stay within the warp once j < 32.
+      if (j > 32) __syncthreads();
+      else if (j > 1) __syncwarp();
+      else __syncthreads();
+    }
+  }
+  for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) p.order[sg.s + i] = s_id[uint32_t(s_word[i])];
+}
+
+// Segments of up to TPS primitives, TPS lanes each, one primitive per lane.
+template <int TPS>
+__global__ void __launch_bounds__(256) level_group_kernel(const LevelParams p) {
+  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / TPS;
+  const uint32_t i = threadIdx.x % TPS;
+  const bool some = g < *p.m;  // every lane stays for the warp's shuffles
+  const Seg sg = some ? p.cur[g] : Seg{0, 0, 0};
+  const uint32_t count = sg.e - sg.s;
+  const uint32_t id = i < count ? p.order[sg.s + i] : 0u;
+  float lo[kMaxDim], hi[kMaxDim], clo[kMaxDim], chi[kMaxDim];
+  empty_box(lo, hi, clo, chi);
+  if (i < count) fold_box(p, id, lo, hi, clo, chi);
+  reduce_lanes<TPS>(p.D, lo, hi, clo, chi);
+  int axis = -1;
+  if (some && i == 0) axis = decide(p, sg, lo, hi, clo, chi);
+  axis = __shfl_sync(0xffffffffu, axis, 0, TPS);
+  if (!__any_sync(0xffffffffu, axis >= 0)) return;
+  unsigned long long w = ~0ull;
+  if (axis >= 0 && i < count) w = ((unsigned long long)p.keys[size_t(axis) * p.n + id] << 32) | i;
+#pragma unroll
+  for (uint32_t k = 2; k <= TPS; k <<= 1) {
+#pragma unroll
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, w, j, TPS);
+      const bool low = (i & j) == 0, up = (i & k) == 0;
+      w = (low == up) ? (w < o ? w : o) : (w < o ? o : w);
+    }
+  }
+  const uint32_t sorted = __shfl_sync(0xffffffffu, id, int(uint32_t(w) & (TPS - 1)), TPS);
+  if (axis >= 0 && i < count) p.order[sg.s + i] = sorted;
 }
 
 // Subtree node counts, one level at a time from the deepest (level L's ids
@@ -365,7 +469,10 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
 
   // Scratch, carved from one stream-ordered allocation.
   sqi::Carve cv;
-  constexpr uint32_t kWide = 1024;  // levels with this many segments or more: one warp per segment
+  // Segments of the top levels (longer than kBlockSort): their reductions.
+  uint32_t top_segs = 1;
+  for (uint32_t L = 0; L < n_levels; ++L)
+    if (longest_at[L] > kBlockSort) top_segs = uint32_t(bound_at(L));
   size_t sort_bytes = 0;
   int pos_bits = 1;
   while (pos_bits < 32 && (uint64_t(1) << pos_bits) < n) ++pos_bits;
@@ -376,7 +483,7 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
   const size_t o_keys = cv.take(size_t(D) * n * 4), o_idx0 = cv.take(size_t(n) * 4), o_idx1 = cv.take(size_t(n) * 4),
                o_sk0 = cv.take(size_t(n) * 8), o_sk1 = cv.take(size_t(n) * 8),
                o_seg0 = cv.take((size_t(n) + 1) * sizeof(Seg)), o_seg1 = cv.take((size_t(n) + 1) * sizeof(Seg)),
-               o_red = cv.take(size_t(kWide) * 4 * kMaxDim * 4), o_axis = cv.take(size_t(kWide) * 4),
+               o_red = cv.take(size_t(top_segs) * 4 * kMaxDim * 4), o_axis = cv.take(size_t(top_segs) * 4),
                o_nodes = cv.take(N2 * sizeof(LNode)), o_lb = cv.take(N2 * 2 * D * 4), o_size = cv.take(N2 * 4),
                o_pre = cv.take(N2 * 4), o_ctr = cv.take(16), o_lv = cv.take(size_t(2) * (n_levels + 1) * 4),
                o_sort = cv.take(sort_bytes);
@@ -419,27 +526,40 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
   uint64_t own_launches = 1;  // keys_kernel
   for (uint32_t L = 0; L < n_levels; ++L) {
     const uint64_t bound = bound_at(L), longest = longest_at[L];
-    const bool may_split = longest > kLeafSize;  // false only on the last level
-    if (may_split) place_keys_kernel<<<std::min<uint32_t>(blocks_for(n, 256), 148 * 8), 256, 0, st>>>(skeys, n);
-    LevelParams p{d_prim_aabbs, D, n, keys, idx, cur, level_info + 2 * L + 1, nxt, ctr, nodes, lbounds, skeys, red,
-                  axis, 4096u};
-    if (bound >= kWide) {
-      level_kernel<32><<<blocks_for(bound, 8), 256, 0, st>>>(p);
-      own_launches += 1;
-    } else {
-      const dim3 grid(uint32_t(std::max<uint64_t>(1, (longest + p.chunk - 1) / p.chunk)), uint32_t(bound));
+    const bool top = longest > kBlockSort;
+    // The shortest segment of the level is at least n >> L long.
+    uint32_t shift = 0;
+    while ((n >> L) >> (shift + 1)) ++shift;
+    LevelParams p{d_prim_aabbs, D, n, keys, idx, cur, level_info + 2 * L + 1, idx, nxt, ctr, nodes, lbounds, skeys, red,
+                  axis, 4096u, uint32_t((longest + 4095) / 4096), shift};
+    if (top) {
+      place_keys_kernel<<<std::min<uint32_t>(blocks_for(n, 256), 148 * 8), 256, 0, st>>>(skeys, n, shift);
+      const uint32_t grid = uint32_t(bound) * p.chunks;
       red_init_kernel<<<blocks_for(bound * 4 * kMaxDim, 256), 256, 0, st>>>(red, uint32_t(bound));
       red_kernel<<<grid, 256, 0, st>>>(p);
       decide_kernel<<<blocks_for(bound, 128), 128, 0, st>>>(p);
       split_keys_kernel<<<grid, 256, 0, st>>>(p);
-      own_launches += 4;
+      own_launches += 5;
+    } else if (longest > 32) {
+      uint32_t padded = 32;
+      while (padded < longest) padded <<= 1;
+      const uint32_t threads = std::min<uint32_t>(256, std::max<uint32_t>(32, padded / 4));
+      level_block_kernel<<<uint32_t(bound), threads, padded * 12, st>>>(p, padded);
+      own_launches += 1;
+    } else if (longest > 8) {
+      level_group_kernel<32><<<blocks_for(bound * 32, 256), 256, 0, st>>>(p);
+      own_launches += 1;
+    } else {
+      level_group_kernel<8><<<blocks_for(bound * 8, 256), 256, 0, st>>>(p);
+      own_launches += 1;
     }
     advance_kernel<<<1, 1, 0, st>>>(ctr, level_info, L);
-    own_launches += 1 + (may_split ? 1 : 0);
+    own_launches += 1;
     CKB(cudaGetLastError());
-    if (may_split) {
+    if (top) {
       size_t need = sort_bytes;
-      CKB(cub::DeviceRadixSort::SortPairs(temp, need, skeys, skeys_alt, idx, idx_alt, int(n), 0, end_bit, st));
+      const int bits = 32 + std::max(pos_bits - int(shift), 1);
+      CKB(cub::DeviceRadixSort::SortPairs(temp, need, skeys, skeys_alt, idx, idx_alt, int(n), 0, bits, st));
       std::swap(idx, idx_alt);
       own_launches += 1;
     }

@@ -116,3 +116,19 @@ def test_device_tree_answers_as_oracle(ctx):
     ref = O.Scene("boxes", 3, s["prims"]).nearest(s["rays"], s["max_toi"])
     assert_same_nearest(ref, got, label="device-built tree")
     scene.close()
+
+
+@pytest.mark.parametrize("dim", [2, 3, 6])
+@pytest.mark.parametrize("n", [8, 32, 64, 65, 2048, 2049, 4096, 8193, 70_001])
+def test_edges_of_the_level_kernels(ctx, n, dim):
+    """Segments around 8 and 32 lanes, the block sort's 2,048 and the radix
+    levels above it; half of the leaves share one centroid, so that long leaf
+    segments end early beside segments that still split."""
+    rng = scenes.Rng(500 + n + dim)
+    b = boxes(rng, n, dim)
+    check(ctx, dim, b, f"n={n}")
+    same = b.copy()
+    same[: n // 2] = b[0]
+    check(ctx, dim, same[np.argsort(rng.take(n), kind="stable")], f"n={n}, half coincident")
+    grid = np.floor(b[:, :dim] / 25.0).astype(np.float32)
+    check(ctx, dim, np.concatenate([grid, grid + 1.0], axis=1), f"n={n}, ties")
