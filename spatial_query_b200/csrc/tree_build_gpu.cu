@@ -81,15 +81,16 @@ __global__ void keys_kernel(const float* __restrict__ aabbs, uint32_t n, int D, 
 
 struct LevelParams {
   const float* aabbs;
+  bool pairs;            // aabbs is 8-byte aligned: read as D two-float loads
   int D;
   uint32_t n;
   const uint32_t* keys;  // [D][n]
   const uint32_t* idx;   // the current primitive order
   const Seg* cur;
-  const uint32_t* m;     // segments of this level (device memory)
+  const uint32_t* m;     // segments of this level (device memory); their first level-order id is m[-1]
   uint32_t* order;       // small segments: the primitive order, sorted in place (same array as idx)
   Seg* next;             // the next level's segments (appended)
-  uint32_t* counters;    // [0] next segments, [1] nodes made, [2] split segments
+  uint32_t* counters;    // [0] next segments, [1] nodes made up to this level
   LNode* nodes;          // by level-order id
   float* bounds;         // by level-order id: min[D], max[D]
   unsigned long long* sort_keys;  // per position: (segment start >> shift) << 32 | split-axis key, or (position >> shift) << 32
@@ -106,50 +107,65 @@ __device__ __forceinline__ float ukey_float(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// Leaf or split of segment sg from its reduced boxes (tree.rs:129-154):
-// writes the node's bounds and record, appends the children's segments,
-// and returns the split axis (-1: leaf). One thread per segment.
-__device__ int decide(const LevelParams& p, const Seg& sg, const float* lo, const float* hi, const float* clo,
-                      const float* chi) {
-  const int D = p.D;
-  const uint32_t count = sg.e - sg.s;
-  float* bo = p.bounds + size_t(sg.node) * 2 * D;
-  for (int k = 0; k < D; ++k) {
-    bo[k] = lo[k];
-    bo[D + k] = hi[k];
-  }
-  LNode nd{sg.s, sg.e, kNone, kNone};
-  int axis = -1;
-  if (count > kLeafSize) {
-    int ax = 0;
-    float ext[kMaxDim];
-    for (int k = 0; k < D; ++k) ext[k] = __fsub_rn(chi[k], clo[k]);
-    for (int k = 1; k < D; ++k)
-      if (ext[k] > ext[ax]) ax = k;
-    if (ext[ax] > kEps) {
-      axis = ax;
-      const uint32_t mid = sg.s + count / 2;
-      const uint32_t c0 = atomicAdd(&p.counters[0], 2u);
-      const uint32_t id0 = atomicAdd(&p.counters[1], 2u);
-      p.next[c0] = Seg{sg.s, mid, id0};
-      p.next[c0 + 1] = Seg{mid, sg.e, id0 + 1};
-      nd.a = id0;
-      nd.b = id0 + 1;
-      atomicAdd(&p.counters[2], 1u);
+// Split axis of a segment of `count` primitives from its reduced centroid box
+// (tree.rs:129-154), -1: a leaf.
+__device__ __forceinline__ int split_axis(int D, uint32_t count, const float* clo, const float* chi) {
+  if (count <= kLeafSize) return -1;
+  int ax = 0;
+  float best = 0.f;
+#pragma unroll
+  for (int k = 0; k < kMaxDim; ++k) {
+    if (k < D) {
+      const float ext = __fsub_rn(chi[k], clo[k]);
+      if (k == 0 || ext > best) {
+        best = ext;
+        ax = k;
+      }
     }
   }
+  return best > kEps ? ax : -1;
+}
+
+// Writes segment sg's bounds and node record and, split, its children's
+// segments at c0 of the next level. Ids are the level's in order: the next
+// level's first id follows this level's last.
+__device__ __forceinline__ void write_node(const LevelParams& p, const Seg& sg, const float* lo, const float* hi, int axis, uint32_t c0) {
+  const int D = p.D;
+  float* bo = p.bounds + size_t(sg.node) * 2 * D;
+#pragma unroll
+  for (int k = 0; k < kMaxDim; ++k) {
+    if (k < D) {
+      bo[k] = lo[k];
+      bo[D + k] = hi[k];
+    }
+  }
+  LNode nd{sg.s, sg.e, kNone, kNone};
+  if (axis >= 0) {
+    const uint32_t mid = sg.s + (sg.e - sg.s) / 2, id0 = p.m[-1] + p.m[0] + c0;
+    p.next[c0] = Seg{sg.s, mid, id0};
+    p.next[c0 + 1] = Seg{mid, sg.e, id0 + 1};
+    nd.a = id0;
+    nd.b = id0 + 1;
+  }
   p.nodes[sg.node] = nd;
+}
+
+// Leaf or split of segment sg by one thread; returns the split axis (-1: leaf).
+__device__ __forceinline__ int decide(const LevelParams& p, const Seg& sg, const float* lo, const float* hi, const float* clo,
+                      const float* chi) {
+  const int axis = split_axis(p.D, sg.e - sg.s, clo, chi);
+  write_node(p, sg, lo, hi, axis, axis >= 0 ? atomicAdd(&p.counters[0], 2u) : 0u);
   return axis;
 }
 
-// Closes level L: the next level's segments were appended with level-order
-// ids [made - count, made); records them and clears the per-level counters.
+// Closes level L: the next level's segments were appended with the level-order
+// ids that follow; records them and clears the level's counter.
 __global__ void advance_kernel(uint32_t* counters, uint32_t* level_info, uint32_t L) {
   const uint32_t m_next = counters[0], made = counters[1];
-  level_info[2 * (L + 1)] = made - m_next;
+  level_info[2 * (L + 1)] = made;
   level_info[2 * (L + 1) + 1] = m_next;
   counters[0] = 0;
-  counters[2] = 0;
+  counters[1] = made + m_next;
 }
 
 // Every position keeps its place unless a split segment claims it.
@@ -164,6 +180,43 @@ __global__ void red_init_kernel(uint32_t* red, uint32_t m) {
   if (i >= m * 4 * kMaxDim) return;
   const uint32_t part = (i / kMaxDim) % 4;  // 0 lo, 1 hi, 2 centroid lo, 3 centroid hi
   red[i] = (part == 0 || part == 2) ? total_ukey(INFINITY) : total_ukey(-INFINITY);
+}
+
+// Folds primitive id's box and centroid into a segment's reduction.
+__device__ __forceinline__ void fold_box(const LevelParams& p, uint32_t id, float* lo, float* hi, float* clo, float* chi) {
+  const float* b = p.aabbs + size_t(id) * 2 * p.D;
+  float v[2 * kMaxDim];  // min[D], max[D]
+  if (p.pairs) {
+#pragma unroll
+    for (int k = 0; k < kMaxDim; ++k) {
+      if (k < p.D) {
+        const float2 x = __ldg(reinterpret_cast<const float2*>(b) + k);
+        v[2 * k] = x.x;
+        v[2 * k + 1] = x.y;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2 * kMaxDim; ++k)
+      if (k < 2 * p.D) v[k] = __ldg(b + k);
+  }
+  // Axis k's bounds are v[k] and v[D + k]: one case per D keeps v in registers.
+  auto axis = [&](int k, float l, float h) {
+    lo[k] = fminf(lo[k], l);
+    hi[k] = fmaxf(hi[k], h);
+    const float c = __fmul_rn(__fadd_rn(l, h), 0.5f);
+    clo[k] = fminf(clo[k], c);
+    chi[k] = fmaxf(chi[k], c);
+  };
+#define SQ_FOLD(DIM)                                  \
+  case DIM:                                           \
+    _Pragma("unroll") for (int k = 0; k < DIM; ++k) axis(k, v[k], v[DIM + k]); \
+    break;
+  switch (p.D) {
+    SQ_FOLD(1) SQ_FOLD(2) SQ_FOLD(3) SQ_FOLD(4) SQ_FOLD(5) SQ_FOLD(6) SQ_FOLD(7) SQ_FOLD(8)
+    default: break;
+  }
+#undef SQ_FOLD
 }
 
 // Top levels: block g * chunks + c reduces positions [s + c * chunk, s + (c + 1)
@@ -182,19 +235,7 @@ __global__ void __launch_bounds__(256) red_kernel(const LevelParams p) {
     lo[k] = clo[k] = INFINITY;
     hi[k] = chi[k] = -INFINITY;
   }
-  for (uint32_t pos = uint32_t(b0) + threadIdx.x; pos < b1; pos += blockDim.x) {
-    const float* b = p.aabbs + size_t(p.idx[pos]) * 2 * D;
-#pragma unroll
-    for (int k = 0; k < kMaxDim; ++k) {
-      if (k < D) {
-        lo[k] = fminf(lo[k], b[k]);
-        hi[k] = fmaxf(hi[k], b[D + k]);
-        const float c = centre(b, D, k);
-        clo[k] = fminf(clo[k], c);
-        chi[k] = fmaxf(chi[k], c);
-      }
-    }
-  }
+  for (uint32_t pos = uint32_t(b0) + threadIdx.x; pos < b1; pos += blockDim.x) fold_box(p, p.idx[pos], lo, hi, clo, chi);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
@@ -246,21 +287,6 @@ __global__ void split_keys_kernel(const LevelParams p) {
   const uint32_t* key = p.keys + size_t(axis) * p.n;
   for (uint32_t pos = uint32_t(b0) + threadIdx.x; pos < b1; pos += blockDim.x)
     p.sort_keys[pos] = ((unsigned long long)(sg.s >> p.shift) << 32) | key[p.idx[pos]];
-}
-
-// Folds primitive id's box and centroid into a segment's reduction.
-__device__ __forceinline__ void fold_box(const LevelParams& p, uint32_t id, float* lo, float* hi, float* clo, float* chi) {
-  const float* b = p.aabbs + size_t(id) * 2 * p.D;
-#pragma unroll
-  for (int k = 0; k < kMaxDim; ++k) {
-    if (k < p.D) {
-      lo[k] = fminf(lo[k], b[k]);
-      hi[k] = fmaxf(hi[k], b[p.D + k]);
-      const float c = centre(b, p.D, k);
-      clo[k] = fminf(clo[k], c);
-      chi[k] = fmaxf(chi[k], c);
-    }
-  }
 }
 
 // The reduction over groups of TPS lanes (min / max are exact in any order).
@@ -373,9 +399,14 @@ __global__ void __launch_bounds__(256) level_group_kernel(const LevelParams p) {
   empty_box(lo, hi, clo, chi);
   if (i < count) fold_box(p, id, lo, hi, clo, chi);
   reduce_lanes<TPS>(p.D, lo, hi, clo, chi);
-  int axis = -1;
-  if (some && i == 0) axis = decide(p, sg, lo, hi, clo, chi);
-  axis = __shfl_sync(0xffffffffu, axis, 0, TPS);
+  // One append per warp for all of its segments that split.
+  const int axis = some ? split_axis(p.D, count, clo, chi) : -1;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t split = __ballot_sync(0xffffffffu, axis >= 0 && i == 0);
+  uint32_t c0 = 0;
+  if (lane == 0 && split) c0 = atomicAdd(&p.counters[0], 2u * __popc(split));
+  c0 = __shfl_sync(0xffffffffu, c0, 0) + 2u * __popc(split & ((1u << lane) - 1u));
+  if (some && i == 0) write_node(p, sg, lo, hi, axis, c0);
   if (!__any_sync(0xffffffffu, axis >= 0)) return;
   unsigned long long w = ~0ull;
   if (axis >= 0 && i < count) w = ((unsigned long long)p.keys[size_t(axis) * p.n + id] << 32) | i;
@@ -413,6 +444,37 @@ __global__ void preorder_kernel(const LNode* __restrict__ nodes, const uint32_t*
   if (nd.a == kNone) return;
   pre[nd.a] = pre[id] + 1;
   pre[nd.b] = pre[id] + 1 + size[nd.a];
+}
+
+// The same for levels [0, top) in one block each (levels of at most kOneBlock
+// nodes: their launches cost more than their work).
+constexpr uint32_t kOneBlock = 1024;
+__global__ void __launch_bounds__(kOneBlock) sizes_top_kernel(const LNode* __restrict__ nodes, const uint32_t* level_info,
+                                                             uint32_t top, uint32_t* size) {
+  for (uint32_t L = top; L-- > 0;) {
+    if (threadIdx.x < level_info[2 * L + 1]) {
+      const uint32_t id = level_info[2 * L] + threadIdx.x;
+      const LNode nd = nodes[id];
+      size[id] = nd.a == kNone ? 1u : 1u + size[nd.a] + size[nd.b];
+    }
+    __syncthreads();
+  }
+}
+__global__ void __launch_bounds__(kOneBlock) preorder_top_kernel(const LNode* __restrict__ nodes, const uint32_t* level_info,
+                                                                uint32_t top, const uint32_t* size, uint32_t* pre) {
+  if (threadIdx.x == 0) pre[0] = 0;
+  __syncthreads();
+  for (uint32_t L = 0; L < top; ++L) {
+    if (threadIdx.x < level_info[2 * L + 1]) {
+      const uint32_t id = level_info[2 * L] + threadIdx.x;
+      const LNode nd = nodes[id];
+      if (nd.a != kNone) {
+        pre[nd.a] = pre[id] + 1;
+        pre[nd.b] = pre[id] + 1 + size[nd.a];
+      }
+    }
+    __syncthreads();
+  }
 }
 
 // The crate's node arrays in preorder (tree::Node: bounds, and either the
@@ -519,7 +581,7 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
   CKB(cudaGetLastError());
   const Seg root{0, n, 0};
   CKB(cudaMemcpyAsync(cur, &root, sizeof(Seg), cudaMemcpyHostToDevice, st));
-  const uint32_t init[4] = {0, 1, 0, 0};  // next segments, nodes made, split segments
+  const uint32_t init[4] = {0, 1, 0, 0};  // next segments, nodes made
   CKB(cudaMemcpyAsync(ctr, init, sizeof(init), cudaMemcpyHostToDevice, st));
   const uint32_t root_level[2] = {0, 1};  // level 0: id 0, one segment
   CKB(cudaMemcpyAsync(level_info, root_level, sizeof(root_level), cudaMemcpyHostToDevice, st));
@@ -530,7 +592,7 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
     // The shortest segment of the level is at least n >> L long.
     uint32_t shift = 0;
     while ((n >> L) >> (shift + 1)) ++shift;
-    LevelParams p{d_prim_aabbs, D, n, keys, idx, cur, level_info + 2 * L + 1, idx, nxt, ctr, nodes, lbounds, skeys, red,
+    LevelParams p{d_prim_aabbs, (reinterpret_cast<uintptr_t>(d_prim_aabbs) & 7) == 0, D, n, keys, idx, cur, level_info + 2 * L + 1, idx, nxt, ctr, nodes, lbounds, skeys, red,
                   axis, 4096u, uint32_t((longest + 4095) / 4096), shift};
     if (top) {
       place_keys_kernel<<<std::min<uint32_t>(blocks_for(n, 256), 148 * 8), 256, 0, st>>>(skeys, n, shift);
@@ -565,10 +627,13 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
     }
     std::swap(cur, nxt);
   }
-  for (uint32_t L = n_levels; L-- > 0;)
+  uint32_t top = 0;
+  while (top < n_levels && bound_at(top) <= kOneBlock) ++top;
+  for (uint32_t L = n_levels; L-- > top;)
     sizes_kernel<<<blocks_for(bound_at(L), 256), 256, 0, st>>>(nodes, level_info, L, size);
-  CKB(cudaMemsetAsync(pre, 0, 4, st));
-  for (uint32_t L = 0; L < n_levels; ++L)
+  sizes_top_kernel<<<1, kOneBlock, 0, st>>>(nodes, level_info, top, size);
+  preorder_top_kernel<<<1, kOneBlock, 0, st>>>(nodes, level_info, top, size, pre);
+  for (uint32_t L = top; L < n_levels; ++L)
     preorder_kernel<<<blocks_for(bound_at(L), 256), 256, 0, st>>>(nodes, level_info, L, size, pre);
   emit_kernel<<<blocks_for(uint64_t(2) * n - 1, 256), 256, 0, st>>>(nodes, lbounds, pre, ctr + 1, node_capacity, D,
                                                                     d_node_bounds, d_child_a, d_child_b, d_prim_count);
@@ -576,7 +641,7 @@ extern "C" int32_t sq_tree_build_d(sq_ctx* ctx, int32_t dim, uint32_t n, const f
   CKB(cudaMemcpyAsync(d_prim_indices, idx, size_t(n) * 4, cudaMemcpyDeviceToDevice, st));
   uint32_t n_nodes = 0;
   CKB(cudaMemcpyAsync(&n_nodes, ctr + 1, 4, cudaMemcpyDeviceToHost, st));
-  ctx->launches += own_launches + 2 * n_levels + 1;
+  ctx->launches += own_launches + 2 * (n_levels - top) + 3;
   int32_t rc = done(SQ_OK);
   CK(cudaStreamSynchronize(st));
   if (n_nodes > node_capacity) return fail(ctx, SQ_ERR_CAPACITY, "node_capacity too small");
