@@ -793,13 +793,20 @@ constexpr uint32_t kOverlapVisitBudget = 128;
 
 // Launches overlap_heavy_kernel over the regions the count pass listed (a
 // block per region, one shared stack of 256 x (depth + 1) entries).
-int32_t launch_heavy(sq_ctx* ctx, const sq_bvh* b, QueryParams& p) {
+// As many blocks as fit the SMs: a region's walk is a chain of fetches and
+// barriers, so resident blocks, not threads, hide it (a launch of the D = 6
+// mixture 179 us at four blocks per SM and a fixed share of the regions each,
+// 137 us as here; 200,000 regions against 1,000,000 boxes 5,536 -> 3,661 us).
+int32_t launch_heavy(sq_ctx* ctx, const sq_bvh* b, QueryParams& p, uint32_t* zeroed_counter) {
   const uint32_t cap = 256u * (b->depth + 1);
   p.stack = int(cap);
+  p.counter = zeroed_counter;
   const size_t smem = size_t(cap) * 4;
   if (smem + kHeavyStage * 4 + 1024 > 48 * 1024) CK(cudaFuncSetAttribute(b->ks.overlap_heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  static_assert(32 * kHeavyWarps == kThreads, "occupancy() counts blocks of kThreads threads");
+  const int bps = occupancy(ctx, b->ks.overlap_heavy, smem);
   void* args[] = {&p};
-  CK(cudaLaunchKernel(b->ks.overlap_heavy, dim3(ctx->sm_count * 4), dim3(32 * kHeavyWarps), args, smem, ctx->stream));
+  CK(cudaLaunchKernel(b->ks.overlap_heavy, dim3(ctx->sm_count * bps), dim3(32 * kHeavyWarps), args, smem, ctx->stream));
   ctx->launches++;
   return SQ_OK;
 }
@@ -825,7 +832,7 @@ int32_t overlap_core(sq_ctx* ctx, const sq_bvh* b, const float* d_regions, uint3
   size_t temp_bytes = scratch_bytes - sc.off;
   CK(cudaMemsetAsync(d_counts, 0, size_t(n + 1) * 4, ctx->stream));
   CK(cudaMemsetAsync(d_hflag, 0, size_t(n) + 1, ctx->stream));
-  CK(cudaMemsetAsync(d_hcount, 0, 8, ctx->stream));  // list count, store cursor
+  CK(cudaMemsetAsync(d_hcount, 0, 16, ctx->stream));  // list count, store cursor, the heavy launches' work counters
   CK(cudaMemsetAsync(d_hstart, 0xFF, size_t(n) * 4, ctx->stream));
   const bool heavy = b->ks.overlap_heavy != nullptr;
   if (b->n_nodes != 0 && n != 0) {
@@ -848,7 +855,7 @@ int32_t overlap_core(sq_ctx* ctx, const sq_bvh* b, const float* d_regions, uint3
     }
     int32_t rc = launch_persistent(ctx, b->ks.overlap, p, b->depth, p.n);
     if (rc) return rc;
-    if (heavy && (rc = launch_heavy(ctx, b, p))) return rc;
+    if (heavy && (rc = launch_heavy(ctx, b, p, d_hcount + 2))) return rc;
   }
   CK(cub::DeviceScan::ExclusiveScan(temp, temp_bytes, d_counts, (unsigned long long*)d_offsets, cuda::std::plus<>{},
                                     0ull, int(n) + 1, ctx->stream));
@@ -880,7 +887,7 @@ int32_t overlap_core(sq_ctx* ctx, const sq_bvh* b, const float* d_regions, uint3
     }
     int32_t rc = launch_persistent(ctx, b->ks.overlap, p, b->depth, p.n);
     if (rc) return rc;
-    if (heavy && hc && (rc = launch_heavy(ctx, b, p))) return rc;
+    if (heavy && hc && (rc = launch_heavy(ctx, b, p, d_hcount + 3))) return rc;
     if ((rc = sort_csr_segments(ctx, d_leaves, tot, d_offsets, n))) return rc;
   }
   return SQ_OK;

@@ -1439,8 +1439,16 @@ __global__ void __launch_bounds__(32 * kHeavyWarps) overlap_heavy_kernel(const Q
   __shared__ uint32_t s_stage[kHeavyStage];
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int cap = p.stack;  // entries
+  __shared__ uint32_t s_next;
   const uint32_t nh = *p.heavy_count & 0x7FFFFFFFu;
-  for (uint32_t i = blockIdx.x; i < nh; i += gridDim.x) {
+  for (;;) {
+    // The next listed region, taken as blocks become free: their walks differ
+    // by orders of magnitude.
+    if (tid == 0) s_next = atomicAdd(p.counter, 1u);
+    __syncthreads();
+    const uint32_t i = s_next;
+    __syncthreads();
+    if (i >= nh) break;
     const uint32_t q = p.heavy_list[i];
     if (!p.fill && p.heavy_flag[q] == 2) continue;  // counted by the count pass (uniform per block)
     if (p.fill && p.heavy_start) {
