@@ -6,12 +6,13 @@
 // bf16 for the tensor cores with f32 master copies for AdamW; every product
 // accumulates in f32. Activations feeding a GEMM are rounded to bf16.
 //
-// Training step on a batch of B rays (B a multiple of 128): the hidden layers
-// forward in one kernel, the output layer with its softmax cross-entropy and
-// gradients in two (guide_ce.cuh), the hidden layers backward in one
-// (guide_hidden.cuh), then AdamW. Products on tcgen05 from tiles that TMA
-// loads; dZ and the activations are transposed by reading their tiles as
-// MN-major operands.
+// Training step on a batch of B rays (B a multiple of 128), as GEMMs
+// C = A * B^T on K-major bf16 operands (guide_gemm.cuh):
+//   Z1 = X W1^T, H1 = relu(Z1 + b1), ..., H3; dZ3 from dH3, dW3 = dZ3^T H2, ...
+// and the output layer (logits, softmax cross-entropy, dH3, dW4, db4) as two
+// kernels that keep the logits in TMEM (guide_ce.cuh). The hidden layers'
+// transposed operands (dZ^T, H^T, W^T) are written by the kernels that produce
+// them.
 //
 // Inference (guide_infer_kernel): one persistent CTA per SM runs the whole
 // network for 256 rays at a time: warp 0 streams pre-swizzled weight chunks
@@ -35,14 +36,12 @@
 
 #include "../../include/sq_guide.h"
 #include "guide_gemm.cuh"
-#include "guide_hidden.cuh"
+#include "guide_ce.cuh"
 #include "sq_internal.cuh"
 
 using namespace sq;
 using namespace sqi;
 using bf16 = __nv_bfloat16;
-using guide::Features;
-using guide::ray_features;
 
 namespace {
 
@@ -50,11 +49,109 @@ constexpr uint32_t kHidden = 128;
 constexpr uint32_t kInputs = 6;
 constexpr uint32_t kInPad = 64;  // layer-1 K padded to one 128-byte panel for the training GEMM
 
-// Where the bf16 copies of the parameters go: weight matrix k is size[k]
-// parameters from offset[k] of the parameter block on.
+// ---------------------------------------------------------------------------
+// Feature map, shared by training and inference: origin to [-1, 1] over the
+// scene box, direction as is. Explicit roundings keep both paths bitwise equal.
+// ---------------------------------------------------------------------------
+struct Features {
+  float lo[3], inv[3];
+};
+
+__device__ __forceinline__ void ray_features(const float* ray, const Features& f, float* x) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    x[i] = __fsub_rn(__fmul_rn(__fmul_rn(__fsub_rn(ray[i], f.lo[i]), f.inv[i]), 2.0f), 1.0f);
+    x[3 + i] = ray[3 + i];
+  }
+}
+
+// X [B x 64] bf16 (zero past the 6 features) and X^T [128 x B] (zero rows past 6).
+__global__ void features_kernel(const float* __restrict__ rays, uint32_t n, uint32_t B, Features f, bf16* X,
+                                bf16* XT) {
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= B) return;
+  float x[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (r < n) ray_features(rays + size_t(r) * 6, f, x);
+  __align__(16) bf16 v[8];
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) v[k] = __float2bfloat16_rn(k < 6 ? x[k] : 0.f);
+  uint4* row = reinterpret_cast<uint4*>(X + size_t(r) * kInPad);
+  row[0] = *reinterpret_cast<const uint4*>(v);
+#pragma unroll
+  for (uint32_t k = 1; k < kInPad / 8; ++k) row[k] = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t k = 0; k < 6; ++k) XT[size_t(k) * B + r] = __float2bfloat16_rn(x[k]);
+}
+
+// H = bf16(relu(Z + b)) and, with HT, H^T, for Z [R x 128] f32.
+__global__ void bias_relu_kernel(const float* __restrict__ Z, const float* __restrict__ b, bf16* H, bf16* HT,
+                                 uint32_t R) {
+  __shared__ bf16 tile[32][33];
+  const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
+    bf16 h = __float2bfloat16_rn(0.f);
+    if (r < R) {
+      h = __float2bfloat16_rn(fmaxf(Z[size_t(r) * kHidden + c] + b[c], 0.f));
+      H[size_t(r) * kHidden + c] = h;
+    }
+    tile[i][threadIdx.x] = h;
+  }
+  if (!HT) return;
+  __syncthreads();
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t c = c0 + i, r = r0 + threadIdx.x;
+    if (r < R) HT[size_t(c) * R + r] = tile[threadIdx.x][i];
+  }
+}
+
+__global__ void count_labels_kernel(const int32_t* __restrict__ labels, uint32_t B, uint32_t n_buckets,
+                                    uint32_t* count) {
+  uint32_t c = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B; i += gridDim.x * blockDim.x)
+    c += (labels[i] >= 0 && uint32_t(labels[i]) < n_buckets) ? 1u : 0u;
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+}
+
+// dZ = bf16(dH * (H > 0)), dZ^T, and db += column sums of dZ.
+__global__ void relu_back_kernel(const float* __restrict__ dH, const bf16* __restrict__ H, bf16* dZ, bf16* dZT,
+                                 float* db, uint32_t R) {
+  __shared__ bf16 tile[32][33];
+  __shared__ float part[8][32];
+  const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  float acc = 0.f;
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
+    bf16 v = __float2bfloat16_rn(0.f);
+    if (r < R) {
+      const size_t k = size_t(r) * kHidden + c;
+      v = __float2bfloat16_rn(__bfloat162float(H[k]) > 0.f ? dH[k] : 0.f);
+      dZ[k] = v;
+    }
+    tile[i][threadIdx.x] = v;
+    acc += __bfloat162float(v);
+  }
+  part[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y == 0) {
+    float t = 0.f;
+    for (uint32_t k = 0; k < blockDim.y; ++k) t += part[k][threadIdx.x];
+    atomicAdd(db + c0 + threadIdx.x, t);
+  }
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t c = c0 + i, r = r0 + threadIdx.x;
+    if (r < R) dZT[size_t(c) * R + r] = tile[threadIdx.x][i];
+  }
+}
+
+// Where the bf16 copies of the parameters go: weight matrix k starts at
+// offset[k] of the parameter block and is rows[k] x cols[k]; its transpose is
+// written where one is kept.
 struct Bf16Copies {
-  size_t offset[4], size[4];
+  size_t offset[4];
+  uint32_t rows[4], cols[4];
   bf16* w[4];
+  bf16* t[4];
 };
 
 // AdamW (decoupled weight decay), as torch.optim.AdamW, and the bf16 copies of
@@ -85,19 +182,27 @@ __global__ void adamw_kernel(float* P, const float* __restrict__ G, float* M, fl
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const size_t j = i - c.offset[k];
-    if (i < c.offset[k] || j >= c.size[k]) continue;
+    if (i < c.offset[k] || j >= size_t(c.rows[k]) * c.cols[k]) continue;
     __align__(8) bf16 w[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) w[e] = __float2bfloat16_rn(p[e]);
     *reinterpret_cast<uint2*>(c.w[k] + j) = *reinterpret_cast<const uint2*>(w);
+    if (c.t[k]) {
+      const uint32_t r = uint32_t(j / c.cols[k]), col = uint32_t(j % c.cols[k]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) c.t[k][size_t(col + e) * c.rows[k] + r] = w[e];
+    }
   }
 }
 
-// bf16 copy of W [rows x cols].
-__global__ void to_bf16_kernel(const float* __restrict__ W, bf16* Wb, uint32_t rows, uint32_t cols) {
+// bf16 copy of W [rows x cols] and, optionally, its transpose [cols x rows].
+__global__ void to_bf16_kernel(const float* __restrict__ W, bf16* Wb, bf16* WbT, uint32_t rows, uint32_t cols) {
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < size_t(rows) * cols;
-       i += size_t(gridDim.x) * blockDim.x)
-    Wb[i] = __float2bfloat16_rn(W[i]);
+       i += size_t(gridDim.x) * blockDim.x) {
+    const bf16 v = __float2bfloat16_rn(W[i]);
+    Wb[i] = v;
+    if (WbT) WbT[(i % cols) * rows + i / cols] = v;
+  }
 }
 
 // Shared-memory images of K-major weight rows, 128-byte swizzled: rows
@@ -125,6 +230,17 @@ __global__ void bucket_of_id_kernel(const uint32_t* __restrict__ prim_ids, const
     else hi = mid;
   }
   out[prim_ids[pos]] = int32_t(lo);
+}
+
+// Batch gather for shuffled epochs: rays and labels of perm[0 .. B).
+__global__ void gather_batch_kernel(const float* __restrict__ rays, const int32_t* __restrict__ labels,
+                                    const uint32_t* __restrict__ perm, uint32_t B, float* b_rays, int32_t* b_labels) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= B) return;
+  const size_t r = perm[i];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) b_rays[size_t(i) * 6 + k] = rays[r * 6 + k];
+  b_labels[i] = labels[r];
 }
 
 __global__ void labels_kernel(const uint32_t* __restrict__ leaf, const int32_t* __restrict__ bucket_of_id,
@@ -489,9 +605,11 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uin
 int* g_err_slot(sq_ctx* ctx);
 
 // C[M x N] = A[M x K] * B[N x K]^T. a_rows / b_rows: allocated rows of A and B
-// (at least M and N; at least one box of 128 rows).
+// (at least M and N; at least one box of 128 rows). into_zeros: C holds zeros,
+// so a product whose tiles leave SMs idle may be split along K, its shares
+// added in the L2.
 int32_t gemm(sq_ctx* ctx, const bf16* A, uint64_t a_rows, uint32_t lda, const bf16* B, uint64_t b_rows, uint32_t ldb,
-             float* C, uint32_t M, uint32_t N, uint32_t K, uint32_t ldc) {
+             float* C, uint32_t M, uint32_t N, uint32_t K, uint32_t ldc, bool into_zeros = false) {
   if (M == 0 || N == 0) return SQ_OK;
   if (K == 0) {
     for (uint32_t r = 0; r < M; ++r) CK(cudaMemsetAsync(C + size_t(r) * ldc, 0, size_t(N) * 4, ctx->stream));
@@ -512,8 +630,14 @@ int32_t gemm(sq_ctx* ctx, const bf16* A, uint64_t a_rows, uint32_t lda, const bf
   int* err = g_err_slot(ctx);
   if (!err) return fail(ctx, SQ_ERR_CUDA, "error slot");
   dim3 grid((M + 127) / 128, (N + BN - 1) / BN);
-  guide::gemm_tn_kernel<BN><<<grid, guide::kGemmThreads, smem, ctx->stream>>>(ta, tb, C, int(M), int(N), int(K),
-                                                                                int(ldc), err);
+  // Shares of at least four K panels (one pipeline's depth), as many as fill
+  // the SMs once. A weight gradient of a hidden layer is one tile with K = the
+  // batch: 128 panels on one SM, 60 us per 8,192 rows; 32 shares take 7 us.
+  const uint32_t panels = (K + 63) / 64, tiles = grid.x * grid.y;
+  const bool split = into_zeros && tiles < uint32_t(ctx->sm_count) && panels >= 8;
+  if (split) grid.z = std::min<uint32_t>(panels / 4, std::max<uint32_t>(uint32_t(ctx->sm_count) / tiles, 1));
+  guide::gemm_tn_kernel<BN><<<grid, guide::kGemmThreads, smem, ctx->stream>>>(
+      ta, tb, C, int(M), int(N), int(K), int(ldc), split ? guide::kEpiReduce : guide::kEpiStore, err);
   ctx->launches++;
   CK(cudaGetLastError());
   return SQ_OK;
@@ -580,8 +704,9 @@ struct sq_guide {
   size_t n_p = 0;
   size_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0, oW4 = 0, ob4 = 0;
   float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;
-  // bf16 weights
+  // bf16 weights and transposes
   bf16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr, *W4b = nullptr;
+  bf16 *W2bT = nullptr, *W3bT = nullptr;
   // inference images and bias
   uint8_t *w1_img = nullptr, *w23_img = nullptr, *w4_img = nullptr;
   float* infer_bias = nullptr;
@@ -593,22 +718,23 @@ struct sq_guide {
   int32_t* d_bucket_of_id = nullptr;
   // batch scratch
   uint32_t B = 0;
-  bf16 *X = nullptr, *H[3] = {};
+  bf16 *X = nullptr, *XT = nullptr, *H[3] = {}, *HT[3] = {}, *dZ = nullptr, *dZT = nullptr;  // HT[2]: not made
   // output layer: shares of the columns per row's statistics, (max, sum) per share half, the label's logit
   uint32_t ce_splits = 1;
   float2* ce_part = nullptr;
   float* ce_zy = nullptr;
-  float *dH = nullptr, *loss = nullptr;  // loss: the batch's sum, then (as u32) its labelled rows
+  float *Z = nullptr, *dH = nullptr, *loss = nullptr;  // loss: the batch's sum, then (as u32) its labelled rows
   uint32_t* count = nullptr;
   std::vector<void*> allocs;
   // label scratch
   uint32_t* d_leaf = nullptr;
   uint32_t leaf_cap = 0;
-  // shuffled training: permutation of the epoch and the batch's gathered labels
+  // shuffled training: permutation of the epoch and the gathered batch
   uint32_t* d_perm = nullptr;
   uint32_t perm_cap = 0;
   float* loss_log = nullptr;  // an epoch's (loss, count) pairs, one per step
   uint32_t log_cap = 0;
+  float* b_rays = nullptr;
   int32_t* b_labels = nullptr;
 };
 
@@ -660,11 +786,11 @@ void build_buckets(const sq_bvh* b, uint32_t depth, std::vector<uint2>& table, s
 int32_t refresh_bf16(sq_guide* g) {
   sq_ctx* ctx = g->ctx;
   const uint32_t T = 256;
-  to_bf16_kernel<<<blocks_for(kHidden * kInPad, T), T, 0, ctx->stream>>>(g->P + g->oW1, g->W1b, kHidden, kInPad);
-  to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW2, g->W2b, kHidden, kHidden);
-  to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW3, g->W3b, kHidden, kHidden);
-  to_bf16_kernel<<<blocks_for(size_t(g->n_out) * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW4, g->W4b, g->n_out,
-                                                                                      kHidden);
+  to_bf16_kernel<<<blocks_for(kHidden * kInPad, T), T, 0, ctx->stream>>>(g->P + g->oW1, g->W1b, nullptr, kHidden, kInPad);
+  to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW2, g->W2b, g->W2bT, kHidden, kHidden);
+  to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW3, g->W3b, g->W3bT, kHidden, kHidden);
+  to_bf16_kernel<<<blocks_for(size_t(g->n_out) * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW4, g->W4b, nullptr,
+                                                                                      g->n_out, kHidden);
   ctx->launches += 4;
   CK(cudaGetLastError());
   g->images_fresh = false;
@@ -768,62 +894,49 @@ int32_t output_layer(sq_guide* g, const int32_t* d_labels) {
   return SQ_OK;
 }
 
-// Forward + backward of one batch (rows perm[i] of the rays and labels, or row
-// i without perm) into g->G; the loss stays on the device.
-int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labels, const uint32_t* d_perm = nullptr) {
+// Forward + backward of one batch into g->G; the mean loss stays on the device.
+int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labels) {
   sq_ctx* ctx = g->ctx;
   const uint32_t B = g->B;
   int32_t rc;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    cudaFuncSetAttribute(guide::hidden_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(guide::FwdSmem::bytes));
-    cudaFuncSetAttribute(guide::hidden_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(guide::BwdSmem::bytes));
-  });
-  int* err = g_err_slot(ctx);
-  if (!err) return fail(ctx, SQ_ERR_CUDA, "error slot");
-  CUtensorMap tw[3], th[3], tx;
-  const bf16* W[3] = {g->W1b, g->W2b, g->W3b};
-  bool maps = make_map(&tx, g->X, B, kInPad, kInPad, 128);
-  for (int l = 0; l < 3; ++l)
-    maps = maps && make_map(&tw[l], W[l], kHidden, l ? kHidden : kInPad, l ? kHidden : kInPad, 128) &&
-           make_map(&th[l], g->H[l], B, kHidden, kHidden, 128);
-  if (!maps) return fail(ctx, SQ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   CK(cudaMemsetAsync(g->G, 0, g->n_p * 4, ctx->stream));
   CK(cudaMemsetAsync(g->loss, 0, 8, ctx->stream));  // and count
+  features_kernel<<<blocks_for(B, 256), 256, 0, ctx->stream>>>(d_rays, B, B, g->feat, g->X, g->XT);
+  count_labels_kernel<<<std::min<uint32_t>(blocks_for(B, 256), 64), 256, 0, ctx->stream>>>(d_labels, B, g->n_buckets,
+                                                                                            g->count);
+  ctx->launches += 2;
+  const dim3 tb(32, 8);
+  const dim3 tgrid(B / 32, kHidden / 32);
+  // forward
+  const bf16* in = g->X;
+  uint32_t in_k = kInPad;
+  const bf16* W[3] = {g->W1b, g->W2b, g->W3b};
+  const size_t ob[3] = {g->ob1, g->ob2, g->ob3};
+  for (int l = 0; l < 3; ++l) {
+    if ((rc = gemm(ctx, in, B, in_k, W[l], kHidden, in_k, g->Z, B, kHidden, in_k, kHidden))) return rc;
+    bias_relu_kernel<<<tgrid, tb, 0, ctx->stream>>>(g->Z, g->P + ob[l], g->H[l], g->HT[l], B);  // H3: no transpose
+    ctx->launches++;
+    in = g->H[l];
+    in_k = kHidden;
+  }
+  // the output layer, its loss and its gradients
   CK(cudaMemsetAsync(g->dH, 0, size_t(B) * kHidden * 4, ctx->stream));
-  guide::HiddenForward f{};
-  f.rays = d_rays;
-  f.labels = d_labels;
-  f.perm = d_perm;
-  f.f = g->feat;
-  f.b[0] = g->P + g->ob1;
-  f.b[1] = g->P + g->ob2;
-  f.b[2] = g->P + g->ob3;
-  f.X = g->X;
-  f.batch_labels = d_perm ? g->b_labels : nullptr;
-  f.count = g->count;
-  f.n_buckets = g->n_buckets;
-  f.err = err;
-  guide::hidden_forward_kernel<<<B / 128, guide::kFwdThreads, guide::FwdSmem::bytes, ctx->stream>>>(
-      tw[0], tw[1], tw[2], th[0], th[1], th[2], f);
-  ctx->launches++;
-  CK(cudaGetLastError());
-  if ((rc = output_layer(g, d_perm ? g->b_labels : d_labels))) return rc;
-  guide::HiddenBackward b{};
-  b.dH3 = g->dH;
-  b.H3 = g->H[2];
-  b.dW[0] = g->G + g->oW1;
-  b.dW[1] = g->G + g->oW2;
-  b.dW[2] = g->G + g->oW3;
-  b.db[0] = g->G + g->ob1;
-  b.db[1] = g->G + g->ob2;
-  b.db[2] = g->G + g->ob3;
-  b.err = err;
-  guide::hidden_backward_kernel<<<B / 128, guide::kCeThreads, guide::BwdSmem::bytes, ctx->stream>>>(
-      th[1], th[0], tx, tw[2], tw[1], b);
-  ctx->launches++;
+  if ((rc = output_layer(g, d_labels))) return rc;
+  // backward
+  const bf16* WT[3] = {nullptr, g->W2bT, g->W3bT};
+  const size_t oW[3] = {g->oW1, g->oW2, g->oW3};
+  for (int l = 2; l >= 0; --l) {
+    relu_back_kernel<<<tgrid, tb, 0, ctx->stream>>>(g->dH, g->H[l], g->dZ, g->dZT, g->G + ob[l], B);
+    ctx->launches++;
+    // dW_l = dZ^T [128 x B] * (input of layer l)^T [K x B]^T
+    const bf16* inT = l == 0 ? g->XT : g->HT[l - 1];
+    const uint32_t K_l = l == 0 ? kInPad : kHidden;
+    if ((rc = gemm(ctx, g->dZT, kHidden, B, inT, kHidden, B, g->G + oW[l], kHidden, K_l, B, K_l, true)))
+      return rc;
+    if (l > 0) {
+      if ((rc = gemm(ctx, g->dZ, B, kHidden, WT[l], kHidden, kHidden, g->dH, B, kHidden, kHidden, kHidden))) return rc;
+    }
+  }
   CK(cudaGetLastError());
   return SQ_OK;
 }
@@ -849,10 +962,11 @@ int32_t adam_step(sq_guide* g) {
   g->steps++;
   const double bc1 = 1.0 - std::pow(double(g->cfg.beta1), double(g->steps));
   const double bc2 = 1.0 - std::pow(double(g->cfg.beta2), double(g->steps));
-  const size_t hh = size_t(kHidden) * kHidden;
   const Bf16Copies c{{g->oW1, g->oW2, g->oW3, g->oW4},
-                     {size_t(kHidden) * kInPad, hh, hh, size_t(g->n_out) * kHidden},
-                     {g->W1b, g->W2b, g->W3b, g->W4b}};
+                     {kHidden, kHidden, kHidden, g->n_out},
+                     {kInPad, kHidden, kHidden, kHidden},
+                     {g->W1b, g->W2b, g->W3b, g->W4b},
+                     {nullptr, g->W2bT, g->W3bT, nullptr}};
   adamw_kernel<<<blocks_for((g->n_p + 3) / 4, 256), 256, 0, ctx->stream>>>(
       g->P, g->G, g->M, g->V, g->n_p, g->cfg.lr, g->cfg.beta1, g->cfg.beta2, g->cfg.eps, g->cfg.weight_decay,
       float(bc1), float(bc2), c);
@@ -982,27 +1096,30 @@ extern "C" int32_t sq_guide_create(sq_ctx* ctx, const sq_bvh* b, const sq_guide_
   if ((rc = A(&g->P, g->n_p * 4)) || (rc = A(&g->G, g->n_p * 4)) || (rc = A(&g->M, g->n_p * 4)) ||
       (rc = A(&g->V, g->n_p * 4)) || (rc = A(&g->W1b, kHidden * kInPad * 2)) ||
       (rc = A(&g->W2b, kHidden * kHidden * 2)) || (rc = A(&g->W3b, kHidden * kHidden * 2)) ||
-      (rc = A(&g->W4b, NO * kHidden * 2)) ||
+      (rc = A(&g->W4b, NO * kHidden * 2)) || (rc = A(&g->W2bT, kHidden * kHidden * 2)) ||
+      (rc = A(&g->W3bT, kHidden * kHidden * 2)) ||
       (rc = A(&g->w1_img, 16384)) || (rc = A(&g->w23_img, 2 * kChunkBytes)) ||
       (rc = A(&g->w4_img, NO / 128 * kChunkBytes)) || (rc = A(&g->infer_bias, (384 + NO) * 4)) ||
       (rc = A(&g->d_buckets, table.size() * sizeof(uint2))) || (rc = A(&g->d_bucket_sibs, sibs.size() * 4)) ||
       (rc = A(&g->d_bucket_of_id, size_t(b->n_prims) * 4)) ||
-      (rc = A(&g->X, B * kInPad * 2)) ||
-      (rc = A(&g->ce_part, B * 2 * g->ce_splits * sizeof(float2))) || (rc = A(&g->ce_zy, B * 4)) ||
+      (rc = A(&g->X, B * kInPad * 2)) || (rc = A(&g->XT, size_t(kHidden) * B * 2)) ||
+      (rc = A(&g->Z, B * kHidden * 4)) ||
+      (rc = A(&g->ce_part, B * 2 * g->ce_splits * sizeof(float2))) || (rc = A(&g->ce_zy, B * 4)) || (rc = A(&g->dZ, B * kHidden * 2)) || (rc = A(&g->dZT, B * kHidden * 2)) ||
       (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) ||
-      (rc = A(&g->b_labels, B * 4))) {
+      (rc = A(&g->b_rays, B * 6 * 4)) || (rc = A(&g->b_labels, B * 4))) {
     sq_guide_destroy(g.release());
     return rc;
   }
   g->count = reinterpret_cast<uint32_t*>(g->loss + 1);
   for (int l = 0; l < 3; ++l)
-    if ((rc = A(&g->H[l], B * kHidden * 2))) {
+    if ((rc = A(&g->H[l], B * kHidden * 2)) || (l < 2 && (rc = A(&g->HT[l], B * kHidden * 2)))) {
       sq_guide_destroy(g.release());
       return rc;
     }
-  // zero: moments
+  // zero: moments, X^T (rows past the features stay zero), padded W1 columns
   CK(cudaMemset(g->M, 0, g->n_p * 4));
   CK(cudaMemset(g->V, 0, g->n_p * 4));
+  CK(cudaMemset(g->XT, 0, size_t(kHidden) * B * 2));
   // bucket table and per-primitive buckets
   CK(cudaMemcpy(g->d_buckets, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(g->d_bucket_sibs, sibs.data(), sibs.size() * 4, cudaMemcpyHostToDevice));
@@ -1169,7 +1286,10 @@ extern "C" int32_t sq_guide_train_d(sq_guide* g, const float* d_rays, const int3
     CK(cudaMemcpyAsync(g->d_perm, perm.data(), size_t(n) * 4, cudaMemcpyHostToDevice, ctx->stream));
     double sum = 0.0;
     for (uint32_t s = 0; s < steps; ++s) {
-      if ((rc = forward_backward(g, d_rays, d_labels, g->d_perm + size_t(s) * g->B))) return rc;
+      gather_batch_kernel<<<blocks_for(g->B, 256), 256, 0, ctx->stream>>>(d_rays, d_labels, g->d_perm + size_t(s) * g->B,
+                                                                          g->B, g->b_rays, g->b_labels);
+      ctx->launches++;
+      if ((rc = forward_backward(g, g->b_rays, g->b_labels))) return rc;
       // Each step's loss stays on the device until the epoch's end: waiting
       // for it here left the GPU idle for 0.1 ms of every step.
       if (loss_per_epoch)

@@ -79,11 +79,6 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
   umma::tma_load_2d(dst + 16384, map, bar, 64, row);
 }
 
-// Adds four consecutive floats at dst (16-byte aligned) in the L2.
-__device__ __forceinline__ void red_add4(float* dst, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // v[j] += b[j] for 64 columns, b in shared memory (16-byte aligned).
 __device__ __forceinline__ void add_bias64(float* v, const float* b) {
 #pragma unroll

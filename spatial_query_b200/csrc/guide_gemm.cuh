@@ -1,11 +1,11 @@
-// The tcgen05 GEMM of sq_gemm_bf16_tn_d:
+// The tcgen05 GEMM the learned guide trains with:
 //   C[M, N] (f32, row-major, ldc) = A[M, K] * B[N, K]^T
 // with A and B bf16, row-major (K contiguous), loaded by TMA as 128-byte
 // swizzled tiles, multiplied by tcgen05.mma (M = 128, N = BN, K = 16 per
 // instruction) into a TMEM accumulator, and written back by four epilogue
 // warps through tcgen05.ld.
 //
-// One CTA per 128 x BN output tile; a 4-stage TMA -> MMA pipeline over K in
+// One CTA per 128 x BN output tile and share of K; a 4-stage TMA -> MMA pipeline over K in
 // 64-element panels: warp 0 lane 0 issues the loads, warp 1 lane 0 issues the
 // MMAs and frees each stage with tcgen05.commit, all four warps drain TMEM.
 // Rows and columns past M, N and K are zero-filled by TMA and masked at the
@@ -27,10 +27,18 @@ template <int BN> struct GemmSmem {
   static constexpr int bytes = kGemmStages * stage + 1024 /* barriers */ + 1024 /* alignment slack */;
 };
 
+// Epilogue modes: plain store, or add into C with reductions in the L2 (for
+// products split along K: the splits' CTAs add into a C zeroed before).
+enum GemmEpi : int { kEpiStore = 0, kEpiReduce = 1 };
+
+__device__ __forceinline__ void red_add4(float* dst, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_tn_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float* __restrict__ C,
-                   int M, int N, int K, int ldc, int* err) {
+                   int M, int N, int K, int ldc, int epi, int* err) {
   using S = GemmSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = umma::smem_u32(smem_raw);
@@ -44,7 +52,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * 128, n0 = blockIdx.y * BN;
-  const int kt_n = (K + 63) / 64;
+  // This CTA's share of the K panels: blockIdx.z of gridDim.z.
+  const int kt_all = (K + 63) / 64, kt_per = (kt_all + int(gridDim.z) - 1) / int(gridDim.z);
+  const int kt_0 = int(blockIdx.z) * kt_per, kt_n = min(kt_all - kt_0, kt_per);
+  if (kt_n <= 0 && gridDim.z > 1) return;  // the last splits of an uneven share
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGemmStages; ++s) {
@@ -74,8 +85,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (*(volatile int*)s_err) break;
       uint8_t* sa = base + s * S::stage;
       umma::mbar_arrive_expect_tx(&full[s], S::stage);
-      umma::tma_load_2d(sa, &ta, &full[s], kt * 64, m0);
-      umma::tma_load_2d(sa + S::a_bytes, &tb, &full[s], kt * 64, n0);
+      umma::tma_load_2d(sa, &ta, &full[s], (kt_0 + kt) * 64, m0);
+      umma::tma_load_2d(sa + S::a_bytes, &tb, &full[s], (kt_0 + kt) * 64, n0);
     }
     *s_issued = kt;
   } else if (warp == 1 && lane == 0) {
@@ -112,7 +123,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (row < M) {
         float* dst = C + size_t(row) * ldc + n0 + c;
         const int lim = N - (n0 + c);
-        if (lim >= 32 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+        if (epi == kEpiReduce) {
+          if (lim >= 32 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) red_add4(dst + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < lim) atomicAdd(dst + j, v[j]);
+          }
+        } else if (lim >= 32 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         } else {
