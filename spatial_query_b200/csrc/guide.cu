@@ -144,54 +144,18 @@ __global__ void relu_back_kernel(const float* __restrict__ dH, const bf16* __res
   }
 }
 
-// Where the bf16 copies of the parameters go: weight matrix k starts at
-// offset[k] of the parameter block and is rows[k] x cols[k]; its transpose is
-// written where one is kept.
-struct Bf16Copies {
-  size_t offset[4];
-  uint32_t rows[4], cols[4];
-  bf16* w[4];
-  bf16* t[4];
-};
-
-// AdamW (decoupled weight decay), as torch.optim.AdamW, and the bf16 copies of
-// the new weights (a pass of their own per matrix cost four launches, 14 us of
-// a step). Four parameters per thread; every matrix starts and ends on a
-// multiple of four.
+// AdamW (decoupled weight decay), as torch.optim.AdamW.
 __global__ void adamw_kernel(float* P, const float* __restrict__ G, float* M, float* V, size_t n, float lr, float b1,
-                             float b2, float eps, float wd, float bc1, float bc2, const Bf16Copies c) {
-  const size_t i = (blockIdx.x * size_t(blockDim.x) + threadIdx.x) * 4;
-  if (i >= n) return;
-  const float4 g4 = *reinterpret_cast<const float4*>(G + i);
-  float4 p4 = *reinterpret_cast<float4*>(P + i), m4 = *reinterpret_cast<float4*>(M + i),
-         v4 = *reinterpret_cast<float4*>(V + i);
-  auto step = [&](float& p, float g, float& m, float& v) {
-    p *= 1.f - lr * wd;
-    m = b1 * m + (1.f - b1) * g;
-    v = b2 * v + (1.f - b2) * g * g;
+                             float b2, float eps, float wd, float bc1, float bc2) {
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+    const float g = G[i];
+    float p = P[i] * (1.f - lr * wd);
+    const float m = b1 * M[i] + (1.f - b1) * g;
+    const float v = b2 * V[i] + (1.f - b2) * g * g;
+    M[i] = m;
+    V[i] = v;
     p -= lr * (m / bc1) / (sqrtf(v / bc2) + eps);
-  };
-  step(p4.x, g4.x, m4.x, v4.x);
-  step(p4.y, g4.y, m4.y, v4.y);
-  step(p4.z, g4.z, m4.z, v4.z);
-  step(p4.w, g4.w, m4.w, v4.w);
-  *reinterpret_cast<float4*>(P + i) = p4;
-  *reinterpret_cast<float4*>(M + i) = m4;
-  *reinterpret_cast<float4*>(V + i) = v4;
-  const float p[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const size_t j = i - c.offset[k];
-    if (i < c.offset[k] || j >= size_t(c.rows[k]) * c.cols[k]) continue;
-    __align__(8) bf16 w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) w[e] = __float2bfloat16_rn(p[e]);
-    *reinterpret_cast<uint2*>(c.w[k] + j) = *reinterpret_cast<const uint2*>(w);
-    if (c.t[k]) {
-      const uint32_t r = uint32_t(j / c.cols[k]), col = uint32_t(j % c.cols[k]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) c.t[k][size_t(col + e) * c.rows[k] + r] = w[e];
-    }
+    P[i] = p;
   }
 }
 
@@ -723,7 +687,7 @@ struct sq_guide {
   uint32_t ce_splits = 1;
   float2* ce_part = nullptr;
   float* ce_zy = nullptr;
-  float *Z = nullptr, *dH = nullptr, *loss = nullptr;  // loss: the batch's sum, then (as u32) its labelled rows
+  float *Z = nullptr, *dH = nullptr, *loss = nullptr;
   uint32_t* count = nullptr;
   std::vector<void*> allocs;
   // label scratch
@@ -732,8 +696,6 @@ struct sq_guide {
   // shuffled training: permutation of the epoch and the gathered batch
   uint32_t* d_perm = nullptr;
   uint32_t perm_cap = 0;
-  float* loss_log = nullptr;  // an epoch's (loss, count) pairs, one per step
-  uint32_t log_cap = 0;
   float* b_rays = nullptr;
   int32_t* b_labels = nullptr;
 };
@@ -900,7 +862,8 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   const uint32_t B = g->B;
   int32_t rc;
   CK(cudaMemsetAsync(g->G, 0, g->n_p * 4, ctx->stream));
-  CK(cudaMemsetAsync(g->loss, 0, 8, ctx->stream));  // and count
+  CK(cudaMemsetAsync(g->loss, 0, 4, ctx->stream));
+  CK(cudaMemsetAsync(g->count, 0, 4, ctx->stream));
   features_kernel<<<blocks_for(B, 256), 256, 0, ctx->stream>>>(d_rays, B, B, g->feat, g->X, g->XT);
   count_labels_kernel<<<std::min<uint32_t>(blocks_for(B, 256), 64), 256, 0, ctx->stream>>>(d_labels, B, g->n_buckets,
                                                                                             g->count);
@@ -941,19 +904,14 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   return SQ_OK;
 }
 
-// The mean loss of a (loss sum, labelled rows) pair.
-float mean_loss(const float* pair) {
-  uint32_t c;
-  std::memcpy(&c, pair + 1, 4);
-  return c ? pair[0] / float(c) : 0.f;
-}
-
 int32_t read_loss(sq_guide* g, float* loss) {
   sq_ctx* ctx = g->ctx;
-  float pair[2];
-  CK(cudaMemcpyAsync(pair, g->loss, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  float s = 0.f;
+  uint32_t c = 0;
+  CK(cudaMemcpyAsync(&s, g->loss, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(&c, g->count, 4, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  *loss = mean_loss(pair);
+  *loss = c ? s / float(c) : 0.f;
   return SQ_OK;
 }
 
@@ -962,18 +920,12 @@ int32_t adam_step(sq_guide* g) {
   g->steps++;
   const double bc1 = 1.0 - std::pow(double(g->cfg.beta1), double(g->steps));
   const double bc2 = 1.0 - std::pow(double(g->cfg.beta2), double(g->steps));
-  const Bf16Copies c{{g->oW1, g->oW2, g->oW3, g->oW4},
-                     {kHidden, kHidden, kHidden, g->n_out},
-                     {kInPad, kHidden, kHidden, kHidden},
-                     {g->W1b, g->W2b, g->W3b, g->W4b},
-                     {nullptr, g->W2bT, g->W3bT, nullptr}};
-  adamw_kernel<<<blocks_for((g->n_p + 3) / 4, 256), 256, 0, ctx->stream>>>(
+  adamw_kernel<<<std::min<uint32_t>(blocks_for(g->n_p, 256), 4096), 256, 0, ctx->stream>>>(
       g->P, g->G, g->M, g->V, g->n_p, g->cfg.lr, g->cfg.beta1, g->cfg.beta2, g->cfg.eps, g->cfg.weight_decay,
-      float(bc1), float(bc2), c);
+      float(bc1), float(bc2));
   ctx->launches++;
   CK(cudaGetLastError());
-  g->images_fresh = false;
-  return SQ_OK;
+  return refresh_bf16(g);
 }
 
 sqi::SeedTable seed_table(const sq_guide* g) {
@@ -1040,7 +992,6 @@ extern "C" int32_t sq_guide_destroy(sq_guide* g) {
   for (void* p : g->allocs) cudaFree(p);  // cudaFree waits for work using the memory
   if (g->d_leaf) cudaFree(g->d_leaf);
   if (g->d_perm) cudaFree(g->d_perm);
-  if (g->loss_log) cudaFree(g->loss_log);
   delete g;
   return SQ_OK;
 }
@@ -1105,12 +1056,11 @@ extern "C" int32_t sq_guide_create(sq_ctx* ctx, const sq_bvh* b, const sq_guide_
       (rc = A(&g->X, B * kInPad * 2)) || (rc = A(&g->XT, size_t(kHidden) * B * 2)) ||
       (rc = A(&g->Z, B * kHidden * 4)) ||
       (rc = A(&g->ce_part, B * 2 * g->ce_splits * sizeof(float2))) || (rc = A(&g->ce_zy, B * 4)) || (rc = A(&g->dZ, B * kHidden * 2)) || (rc = A(&g->dZT, B * kHidden * 2)) ||
-      (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) ||
+      (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) || (rc = A(&g->count, 16)) ||
       (rc = A(&g->b_rays, B * 6 * 4)) || (rc = A(&g->b_labels, B * 4))) {
     sq_guide_destroy(g.release());
     return rc;
   }
-  g->count = reinterpret_cast<uint32_t*>(g->loss + 1);
   for (int l = 0; l < 3; ++l)
     if ((rc = A(&g->H[l], B * kHidden * 2)) || (l < 2 && (rc = A(&g->HT[l], B * kHidden * 2)))) {
       sq_guide_destroy(g.release());
@@ -1264,16 +1214,7 @@ extern "C" int32_t sq_guide_train_d(sq_guide* g, const float* d_rays, const int3
     CK(cudaMalloc(&g->d_perm, size_t(n) * 4));
     g->perm_cap = n;
   }
-  if (loss_per_epoch && g->log_cap < steps) {
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (g->loss_log) CK(cudaFree(g->loss_log));
-    g->loss_log = nullptr;
-    g->log_cap = 0;
-    CK(cudaMalloc(&g->loss_log, size_t(steps) * 8));
-    g->log_cap = steps;
-  }
   std::vector<uint32_t> perm(n);
-  std::vector<float> log(size_t(steps) * 2);
   for (uint32_t e = 0; e < epochs; ++e) {
     // A fresh shuffle per epoch (Fisher-Yates on SplitMix64, seeded by the
     // config seed and the optimiser step), so batches mix both ray kinds.
@@ -1290,16 +1231,12 @@ extern "C" int32_t sq_guide_train_d(sq_guide* g, const float* d_rays, const int3
                                                                           g->B, g->b_rays, g->b_labels);
       ctx->launches++;
       if ((rc = forward_backward(g, g->b_rays, g->b_labels))) return rc;
-      // Each step's loss stays on the device until the epoch's end: waiting
-      // for it here left the GPU idle for 0.1 ms of every step.
-      if (loss_per_epoch)
-        CK(cudaMemcpyAsync(g->loss_log + size_t(s) * 2, g->loss, 8, cudaMemcpyDeviceToDevice, ctx->stream));
+      if (loss_per_epoch) {
+        float l = 0.f;
+        if ((rc = read_loss(g, &l))) return rc;
+        sum += l;
+      }
       if ((rc = adam_step(g))) return rc;
-    }
-    if (loss_per_epoch && steps) {
-      CK(cudaMemcpyAsync(log.data(), g->loss_log, size_t(steps) * 8, cudaMemcpyDeviceToHost, ctx->stream));
-      CK(cudaStreamSynchronize(ctx->stream));
-      for (uint32_t s = 0; s < steps; ++s) sum += mean_loss(log.data() + size_t(s) * 2);
     }
     if (loss_per_epoch) loss_per_epoch[e] = steps ? float(sum / steps) : 0.f;
   }
