@@ -25,8 +25,6 @@
 namespace sq {
 namespace guide {
 
-using bf16 = __nv_bfloat16;
-
 constexpr int kCeThreads = 320;  // warps 0..7 epilogue, warp 8 loads, warp 9 issues MMAs
 constexpr uint32_t kTile = 32768;
 
@@ -77,48 +75,6 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
   umma::mbar_arrive_expect_tx(bar, kTile);
   umma::tma_load_2d(dst, map, bar, 0, row);
   umma::tma_load_2d(dst + 16384, map, bar, 64, row);
-}
-
-// v[j] += b[j] for 64 columns, b in shared memory (16-byte aligned).
-__device__ __forceinline__ void add_bias64(float* v, const float* b) {
-#pragma unroll
-  for (int j = 0; j < 64; j += 4) {
-    const float4 x = *reinterpret_cast<const float4*>(b + j);
-    v[j] += x.x;
-    v[j + 1] += x.y;
-    v[j + 2] += x.z;
-    v[j + 3] += x.w;
-  }
-}
-
-// Adds a warp's 32 rows x 64 columns (lane = row) into rows of 128 floats at
-// dst in global memory. Through a padded shared-memory buffer of the warp, 16
-// rows x 32 columns at a time, so that each reduction instruction covers four
-// whole 128-byte lines instead of a piece of 32 rows (80 -> 68 us per 8,192
-// x 4,096 gradient).
-constexpr int kStageStride = 36;
-constexpr uint32_t kStageBytes = 16 * kStageStride * 4;
-__device__ __forceinline__ void add_rows(float* stage, const float* v, float* dst, int lane) {
-#pragma unroll
-  for (int cb = 0; cb < 64; cb += 32) {
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      __syncwarp();
-      if ((lane >> 4) == half) {
-#pragma unroll
-        for (int k = 0; k < 32; k += 4)
-          *reinterpret_cast<float4*>(stage + (lane & 15) * kStageStride + k) =
-              make_float4(v[cb + k], v[cb + k + 1], v[cb + k + 2], v[cb + k + 3]);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) {
-        const int r = k + (lane >> 3), c = (lane & 7) * 4;
-        const float4 x = *reinterpret_cast<const float4*>(stage + r * kStageStride + c);
-        red_add4(dst + size_t(half * 16 + r) * 128 + cb + c, x.x, x.y, x.z, x.w);
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -219,15 +175,13 @@ __global__ void __launch_bounds__(kCeThreads, 1)
       __syncwarp();
       if (lane == 0) umma::mbar_arrive(&z_empty[z]);
       const uint32_t col = (c0 + i) * 128 + half * 64;  // of v[0]
-      add_bias64(v, s_bias + i * 128 + half * 64);
-      if (col + 64 > p.n_buckets) {
-#pragma unroll
-        for (uint32_t j = 0; j < 64; ++j)
-          if (col + j >= p.n_buckets) v[j] = -INFINITY;
-      }
+      const float* b = s_bias + i * 128 + half * 64;
       float top = -INFINITY;
 #pragma unroll
-      for (uint32_t j = 0; j < 64; ++j) top = fmaxf(top, v[j]);
+      for (uint32_t j = 0; j < 64; ++j) {
+        v[j] = col + j < p.n_buckets ? v[j] + b[j] : -INFINITY;
+        top = fmaxf(top, v[j]);
+      }
       if (y >= int32_t(col) && y < int32_t(col + 64)) {
 #pragma unroll
         for (uint32_t j = 0; j < 64; ++j)
@@ -277,8 +231,7 @@ struct CeGradSmem {
   static constexpr uint32_t h = 2 * kTile;     // 2 slots
   static constexpr uint32_t dz = 4 * kTile;    // one tile per chunk
   static constexpr uint32_t bias = 6 * kTile;  // 256 floats
-  static constexpr uint32_t stage = bias + 1024;  // one per epilogue warp
-  static constexpr uint32_t bars = stage + 8 * kStageBytes;
+  static constexpr uint32_t bars = bias + 1024;
   static constexpr uint32_t bytes = bars + 256 + 1024;
 };
 
@@ -381,14 +334,12 @@ __global__ void __launch_bounds__(kCeThreads, 1)
     const uint32_t q = warp & 3, half = warp >> 2;
     const uint32_t r = q * 32 + lane;  // row of the tile; dW: column of the chunk
     const uint32_t lanes = (q * 32u) << 16;
-    float* stage = reinterpret_cast<float*>(base + CeGradSmem::stage + warp * kStageBytes);
     const float inv_n = 1.0f / float(max(*p.count, 1u));
     // Column sums: this thread adds columns 2 cp and 2 cp + 1 of rows [32 rg, +32) of each dZ tile.
     const uint32_t cp = threadIdx.x & 63, rg = threadIdx.x >> 6;
     float cs[4] = {0.f, 0.f, 0.f, 0.f};
-    float m = 0.f, inv_s = 0.f, scale = 0.f;  // scale: of a labelled row's exponentials, 0 for the others
+    float m = 0.f, inv_s = 0.f;
     int32_t y = -1;
-    uint32_t row = 0;
     // dH of tile t: this thread's row, 64 of its 128 columns, added in the L2.
     auto flush_dh = [&](uint32_t t) -> bool {
       if (!__all_sync(0xffffffffu, wait(dh_full, t & 1, 7))) return false;
@@ -399,7 +350,9 @@ __global__ void __launch_bounds__(kCeThreads, 1)
       umma::tc_fence_before();
       __syncwarp();
       if (lane == 0) umma::mbar_arrive(dh_empty);
-      add_rows(stage, v, p.dH + (size_t(t0 + t) * 128 + q * 32) * 128 + half * 64, lane);
+      float* dst = p.dH + (size_t(t0 + t) * 128 + r) * 128 + half * 64;
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) red_add4(dst + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
       return true;
     };
     // After a wait that gave up (ok false) the warps still meet at every
@@ -409,7 +362,7 @@ __global__ void __launch_bounds__(kCeThreads, 1)
       const uint32_t t = i / nc, c = i % nc;
       if (c == 0) {
         // This row's maximum and sum over all columns, from the shares.
-        row = (t0 + t) * 128 + r;
+        const uint32_t row = (t0 + t) * 128 + r;
         y = p.labels[row];
         if (uint32_t(y) >= p.n_buckets) y = -1;
         const float2* part = p.part + size_t(row) * 2 * p.splits;
@@ -419,7 +372,6 @@ __global__ void __launch_bounds__(kCeThreads, 1)
         for (uint32_t k = 0; k < 2 * p.splits; ++k)
           if (part[k].x > -INFINITY) s += part[k].y * expf(part[k].x - m);
         inv_s = 1.0f / s;
-        scale = y >= 0 ? inv_s * inv_n : 0.f;
         if (blockIdx.x == 0 && half == 0) {
           float l = y >= 0 ? logf(s) + m - p.zy[row] : 0.f;
 #pragma unroll
@@ -439,25 +391,25 @@ __global__ void __launch_bounds__(kCeThreads, 1)
         // The tile of this chunk's last dZ is free once its products are done.
         ok = t == 0 || __all_sync(0xffffffffu, wait(&dz_empty[c], (t - 1) & 1, 9));
         const uint32_t col = (chunk0 + c) * 128 + half * 64;
-        add_bias64(v, s_bias + c * 128 + half * 64);
+        const float* b = s_bias + c * 128 + half * 64;
         uint8_t* panel = base + CeGradSmem::dz + c * kTile + half * 16384;
         if (ok) {
 #pragma unroll
           for (uint32_t j = 0; j < 64; j += 8) {
             __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
-            for (uint32_t k = 0; k < 8; k += 2)
-              o[k / 2] = __floats2bfloat162_rn(expf(v[j + k] - m) * scale, expf(v[j + k + 1] - m) * scale);
+            for (uint32_t k = 0; k < 8; k += 2) {
+              float g[2];
+#pragma unroll
+              for (uint32_t e = 0; e < 2; ++e) {
+                const uint32_t x = col + j + k + e;
+                g[e] = expf(v[j + k + e] + b[j + k + e] - m) * inv_s - (x == uint32_t(y) ? 1.f : 0.f);
+                g[e] = (y >= 0 && x < p.n_buckets) ? g[e] * inv_n : 0.f;
+              }
+              o[k / 2] = __floats2bfloat162_rn(g[0], g[1]);
+            }
             *reinterpret_cast<uint4*>(panel + umma::sw128_offset(r, j)) = *reinterpret_cast<const uint4*>(o);
           }
-          // The label's own column, and the columns past the last bucket.
-          bf16* own = reinterpret_cast<bf16*>(panel);
-          if (y >= int32_t(col) && y < int32_t(col + 64)) {
-            const uint32_t j = uint32_t(y) - col;
-            own[umma::sw128_offset(r, j) / 2] = __float2bfloat16_rn((expf(p.zy[row] - m) * inv_s - 1.f) * inv_n);
-          }
-          for (uint32_t j = p.n_buckets > col ? p.n_buckets - col : 0u; j < 64; ++j)
-            own[umma::sw128_offset(r, j) / 2] = __float2bfloat16_rn(0.f);
           umma::fence_proxy_async();
         }
       }
@@ -488,10 +440,12 @@ __global__ void __launch_bounds__(kCeThreads, 1)
     if (ok && n && __all_sync(0xffffffffu, wait(dw_full, 0, 10))) {
       umma::tc_fence_after();
       for (uint32_t c = 0; c < nc; ++c) {
+        float* dst = p.dW + (size_t(chunk0 + c) * 128 + r) * 128 + half * 64;
         float v[64];
         umma::tmem_ld32(tdw + lanes + c * 128 + half * 64, v);
         umma::tmem_ld32(tdw + lanes + c * 128 + half * 64 + 32, v + 32);
-        add_rows(stage, v, p.dW + (size_t(chunk0 + c) * 128 + q * 32) * 128 + half * 64, lane);
+#pragma unroll
+        for (int j = 0; j < 64; j += 4) red_add4(dst + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
         atomicAdd(p.db + (chunk0 + c) * 128 + 2 * cp, c == 0 ? cs[0] : cs[2]);
         atomicAdd(p.db + (chunk0 + c) * 128 + 2 * cp + 1, c == 0 ? cs[1] : cs[3]);
       }
