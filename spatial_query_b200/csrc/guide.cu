@@ -8,11 +8,10 @@
 //
 // Training step on a batch of B rays (B a multiple of 128), as GEMMs
 // C = A * B^T on K-major bf16 operands (guide_gemm.cuh):
-//   Z1 = X W1^T, H1 = relu(Z1 + b1), ..., H3; dZ3 from dH3, dW3 = dZ3^T H2, ...
-// and the output layer (logits, softmax cross-entropy, dH3, dW4, db4) as two
-// kernels that keep the logits in TMEM (guide_ce.cuh). The hidden layers'
-// transposed operands (dZ^T, H^T, W^T) are written by the kernels that produce
-// them.
+//   Z1 = X W1^T, H1 = relu(Z1 + b1), ..., Z4 = H3 W4^T, softmax cross-entropy
+//   dZ4 = (softmax - onehot) / n_labelled, dW4 = dZ4^T H3, dH3 = dZ4 W4, ...
+// The transposed operands (dZ^T, H^T, W^T) are written by the kernels that
+// produce them.
 //
 // Inference (guide_infer_kernel): one persistent CTA per SM runs the whole
 // network for 256 rays at a time: warp 0 streams pre-swizzled weight chunks
@@ -36,7 +35,6 @@
 
 #include "../../include/sq_guide.h"
 #include "guide_gemm.cuh"
-#include "guide_ce.cuh"
 #include "sq_internal.cuh"
 
 using namespace sq;
@@ -82,7 +80,7 @@ __global__ void features_kernel(const float* __restrict__ rays, uint32_t n, uint
   for (uint32_t k = 0; k < 6; ++k) XT[size_t(k) * B + r] = __float2bfloat16_rn(x[k]);
 }
 
-// H = bf16(relu(Z + b)) and, with HT, H^T, for Z [R x 128] f32.
+// H = bf16(relu(Z + b)) and H^T, for Z [R x 128] f32.
 __global__ void bias_relu_kernel(const float* __restrict__ Z, const float* __restrict__ b, bf16* H, bf16* HT,
                                  uint32_t R) {
   __shared__ bf16 tile[32][33];
@@ -96,7 +94,6 @@ __global__ void bias_relu_kernel(const float* __restrict__ Z, const float* __res
     }
     tile[i][threadIdx.x] = h;
   }
-  if (!HT) return;
   __syncthreads();
   for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
     const uint32_t c = c0 + i, r = r0 + threadIdx.x;
@@ -111,6 +108,73 @@ __global__ void count_labels_kernel(const int32_t* __restrict__ labels, uint32_t
     c += (labels[i] >= 0 && uint32_t(labels[i]) < n_buckets) ? 1u : 0u;
   for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+}
+
+// One row of logits per block: softmax cross-entropy against the label
+// (-1: ignored), dZ = (softmax - onehot) / n_labelled as bf16.
+__global__ void softmax_ce_kernel(const float* __restrict__ Z, const float* __restrict__ b,
+                                  const int32_t* __restrict__ labels, uint32_t n_out, uint32_t n_buckets,
+                                  const uint32_t* count, bf16* dZ, float* loss_sum) {
+  const uint32_t row = blockIdx.x;
+  const float* z = Z + size_t(row) * n_out;
+  bf16* dz = dZ + size_t(row) * n_out;
+  const int32_t y = labels[row];
+  __shared__ float red[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (y < 0 || uint32_t(y) >= n_buckets) {
+    for (uint32_t j = threadIdx.x; j < n_out; j += blockDim.x) dz[j] = __float2bfloat16_rn(0.f);
+    return;
+  }
+  float m = -INFINITY;
+  for (uint32_t j = threadIdx.x; j < n_buckets; j += blockDim.x) m = fmaxf(m, z[j] + b[j]);
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) red[warp] = m;
+  __syncthreads();
+  m = red[0];
+  for (int w = 1; w < nw; ++w) m = fmaxf(m, red[w]);
+  __syncthreads();
+  float s = 0.f;
+  for (uint32_t j = threadIdx.x; j < n_buckets; j += blockDim.x) s += expf(z[j] + b[j] - m);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) red[warp] = s;
+  __syncthreads();
+  s = 0.f;
+  for (int w = 0; w < nw; ++w) s += red[w];
+  const float inv_n = 1.0f / float(max(*count, 1u));
+  const float inv_s = 1.0f / s;
+  for (uint32_t j = threadIdx.x; j < n_out; j += blockDim.x) {
+    float g = 0.f;
+    if (j < n_buckets) g = expf(z[j] + b[j] - m) * inv_s - (j == uint32_t(y) ? 1.f : 0.f);
+    dz[j] = __float2bfloat16_rn(g * inv_n);
+  }
+  if (threadIdx.x == 0) atomicAdd(loss_sum, logf(s) + m - (z[y] + b[y]));
+}
+
+// out[C x R] = in[R x C]^T (bf16), and colsum[c] += sum over rows of in[., c].
+__global__ void transpose_colsum_kernel(const bf16* __restrict__ in, bf16* out, float* colsum, uint32_t R,
+                                        uint32_t C) {
+  __shared__ bf16 tile[32][33];
+  __shared__ float part[8][32];
+  const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  float acc = 0.f;
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
+    bf16 v = __float2bfloat16_rn(0.f);
+    if (r < R && c < C) v = in[size_t(r) * C + c];
+    tile[i][threadIdx.x] = v;
+    acc += __bfloat162float(v);
+  }
+  part[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (colsum && threadIdx.y == 0 && c0 + threadIdx.x < C) {
+    float t = 0.f;
+    for (uint32_t k = 0; k < blockDim.y; ++k) t += part[k][threadIdx.x];
+    atomicAdd(colsum + c0 + threadIdx.x, t);
+  }
+  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
+    const uint32_t c = c0 + i, r = r0 + threadIdx.x;
+    if (r < R && c < C) out[size_t(c) * R + r] = tile[threadIdx.x][i];
+  }
 }
 
 // dZ = bf16(dH * (H > 0)), dZ^T, and db += column sums of dZ.
@@ -670,7 +734,7 @@ struct sq_guide {
   float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;
   // bf16 weights and transposes
   bf16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr, *W4b = nullptr;
-  bf16 *W2bT = nullptr, *W3bT = nullptr;
+  bf16 *W2bT = nullptr, *W3bT = nullptr, *W4bT = nullptr;
   // inference images and bias
   uint8_t *w1_img = nullptr, *w23_img = nullptr, *w4_img = nullptr;
   float* infer_bias = nullptr;
@@ -682,11 +746,8 @@ struct sq_guide {
   int32_t* d_bucket_of_id = nullptr;
   // batch scratch
   uint32_t B = 0;
-  bf16 *X = nullptr, *XT = nullptr, *H[3] = {}, *HT[3] = {}, *dZ = nullptr, *dZT = nullptr;  // HT[2]: not made
-  // output layer: shares of the columns per row's statistics, (max, sum) per share half, the label's logit
-  uint32_t ce_splits = 1;
-  float2* ce_part = nullptr;
-  float* ce_zy = nullptr;
+  bf16 *X = nullptr, *XT = nullptr, *H[3] = {}, *HT[3] = {}, *dZ4 = nullptr, *dZ4T = nullptr, *dZ = nullptr,
+       *dZT = nullptr;
   float *Z = nullptr, *dH = nullptr, *loss = nullptr;
   uint32_t* count = nullptr;
   std::vector<void*> allocs;
@@ -751,7 +812,7 @@ int32_t refresh_bf16(sq_guide* g) {
   to_bf16_kernel<<<blocks_for(kHidden * kInPad, T), T, 0, ctx->stream>>>(g->P + g->oW1, g->W1b, nullptr, kHidden, kInPad);
   to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW2, g->W2b, g->W2bT, kHidden, kHidden);
   to_bf16_kernel<<<blocks_for(kHidden * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW3, g->W3b, g->W3bT, kHidden, kHidden);
-  to_bf16_kernel<<<blocks_for(size_t(g->n_out) * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW4, g->W4b, nullptr,
+  to_bf16_kernel<<<blocks_for(size_t(g->n_out) * kHidden, T), T, 0, ctx->stream>>>(g->P + g->oW4, g->W4b, g->W4bT,
                                                                                       g->n_out, kHidden);
   ctx->launches += 4;
   CK(cudaGetLastError());
@@ -818,48 +879,10 @@ void dev_to_host(const sq_guide* g, const std::vector<float>& d, float* h) {
   copy(g->ob4, g->n_out);
 }
 
-// The output layer of a batch from H3 (guide_ce.cuh): loss, dH3, dW4, db4.
-int32_t output_layer(sq_guide* g, const int32_t* d_labels) {
-  sq_ctx* ctx = g->ctx;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    cudaFuncSetAttribute(guide::ce_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(guide::CeStatsSmem::bytes));
-    cudaFuncSetAttribute(guide::ce_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(guide::CeGradSmem::bytes));
-  });
-  CUtensorMap th, tw;
-  if (!make_map(&th, g->H[2], g->B, kHidden, kHidden, 128) || !make_map(&tw, g->W4b, g->n_out, kHidden, kHidden, 128))
-    return fail(ctx, SQ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-  guide::CeParams p;
-  p.bias = g->P + g->ob4;
-  p.labels = d_labels;
-  p.count = g->count;
-  p.part = g->ce_part;
-  p.zy = g->ce_zy;
-  p.loss = g->loss;
-  p.dH = g->dH;
-  p.dW = g->G + g->oW4;
-  p.db = g->G + g->ob4;
-  p.B = g->B;
-  p.n_chunks = g->n_out / 128;
-  p.n_buckets = g->n_buckets;
-  p.splits = g->ce_splits;
-  p.err = g_err_slot(ctx);
-  if (!p.err) return fail(ctx, SQ_ERR_CUDA, "error slot");
-  const uint32_t tiles = g->B / 128, pairs = (p.n_chunks + 1) / 2;
-  const uint32_t shares = std::min(tiles, std::max<uint32_t>(uint32_t(ctx->sm_count) / pairs, 1));
-  guide::ce_stats_kernel<<<dim3(tiles, p.splits), guide::kCeThreads, guide::CeStatsSmem::bytes, ctx->stream>>>(th, tw, p);
-  guide::ce_grad_kernel<<<dim3(pairs, shares), guide::kCeThreads, guide::CeGradSmem::bytes, ctx->stream>>>(th, tw, p);
-  ctx->launches += 2;
-  CK(cudaGetLastError());
-  return SQ_OK;
-}
-
 // Forward + backward of one batch into g->G; the mean loss stays on the device.
 int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labels) {
   sq_ctx* ctx = g->ctx;
-  const uint32_t B = g->B;
+  const uint32_t B = g->B, NO = g->n_out;
   int32_t rc;
   CK(cudaMemsetAsync(g->G, 0, g->n_p * 4, ctx->stream));
   CK(cudaMemsetAsync(g->loss, 0, 4, ctx->stream));
@@ -877,15 +900,21 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   const size_t ob[3] = {g->ob1, g->ob2, g->ob3};
   for (int l = 0; l < 3; ++l) {
     if ((rc = gemm(ctx, in, B, in_k, W[l], kHidden, in_k, g->Z, B, kHidden, in_k, kHidden))) return rc;
-    bias_relu_kernel<<<tgrid, tb, 0, ctx->stream>>>(g->Z, g->P + ob[l], g->H[l], g->HT[l], B);  // H3: no transpose
+    bias_relu_kernel<<<tgrid, tb, 0, ctx->stream>>>(g->Z, g->P + ob[l], g->H[l], g->HT[l], B);
     ctx->launches++;
     in = g->H[l];
     in_k = kHidden;
   }
-  // the output layer, its loss and its gradients
-  CK(cudaMemsetAsync(g->dH, 0, size_t(B) * kHidden * 4, ctx->stream));
-  if ((rc = output_layer(g, d_labels))) return rc;
+  if ((rc = gemm(ctx, g->H[2], B, kHidden, g->W4b, NO, kHidden, g->Z, B, NO, kHidden, NO))) return rc;
+  softmax_ce_kernel<<<B, 256, 0, ctx->stream>>>(g->Z, g->P + g->ob4, d_labels, NO, g->n_buckets, g->count, g->dZ4,
+                                                g->loss);
+  transpose_colsum_kernel<<<dim3(B / 32, NO / 32), tb, 0, ctx->stream>>>(g->dZ4, g->dZ4T, g->G + g->ob4, B, NO);
+  ctx->launches += 2;
   // backward
+  if ((rc = gemm(ctx, g->dZ4T, NO, B, g->HT[2], kHidden, B, g->G + g->oW4, NO, kHidden, B, kHidden, true)))
+    return rc;
+  CK(cudaMemsetAsync(g->dH, 0, size_t(B) * kHidden * 4, ctx->stream));
+  if ((rc = gemm(ctx, g->dZ4, B, NO, g->W4bT, kHidden, NO, g->dH, B, kHidden, NO, kHidden, true))) return rc;
   const bf16* WT[3] = {nullptr, g->W2bT, g->W3bT};
   const size_t oW[3] = {g->oW1, g->oW2, g->oW3};
   for (int l = 2; l >= 0; --l) {
@@ -1043,26 +1072,25 @@ extern "C" int32_t sq_guide_create(sq_ctx* ctx, const sq_bvh* b, const sq_guide_
   int32_t rc;
   auto A = [&](auto** p, size_t bytes) { return galloc(gp, reinterpret_cast<void**>(p), bytes); };
   const size_t NO = g->n_out, B = g->B;
-  g->ce_splits = std::min<uint32_t>(g->n_out / 128, std::max<uint32_t>(uint32_t(ctx->sm_count) / (g->B / 128), 1));
   if ((rc = A(&g->P, g->n_p * 4)) || (rc = A(&g->G, g->n_p * 4)) || (rc = A(&g->M, g->n_p * 4)) ||
       (rc = A(&g->V, g->n_p * 4)) || (rc = A(&g->W1b, kHidden * kInPad * 2)) ||
       (rc = A(&g->W2b, kHidden * kHidden * 2)) || (rc = A(&g->W3b, kHidden * kHidden * 2)) ||
       (rc = A(&g->W4b, NO * kHidden * 2)) || (rc = A(&g->W2bT, kHidden * kHidden * 2)) ||
-      (rc = A(&g->W3bT, kHidden * kHidden * 2)) ||
+      (rc = A(&g->W3bT, kHidden * kHidden * 2)) || (rc = A(&g->W4bT, NO * kHidden * 2)) ||
       (rc = A(&g->w1_img, 16384)) || (rc = A(&g->w23_img, 2 * kChunkBytes)) ||
       (rc = A(&g->w4_img, NO / 128 * kChunkBytes)) || (rc = A(&g->infer_bias, (384 + NO) * 4)) ||
       (rc = A(&g->d_buckets, table.size() * sizeof(uint2))) || (rc = A(&g->d_bucket_sibs, sibs.size() * 4)) ||
       (rc = A(&g->d_bucket_of_id, size_t(b->n_prims) * 4)) ||
       (rc = A(&g->X, B * kInPad * 2)) || (rc = A(&g->XT, size_t(kHidden) * B * 2)) ||
-      (rc = A(&g->Z, B * kHidden * 4)) ||
-      (rc = A(&g->ce_part, B * 2 * g->ce_splits * sizeof(float2))) || (rc = A(&g->ce_zy, B * 4)) || (rc = A(&g->dZ, B * kHidden * 2)) || (rc = A(&g->dZT, B * kHidden * 2)) ||
+      (rc = A(&g->Z, B * std::max<size_t>(NO, kHidden) * 4)) || (rc = A(&g->dZ4, B * NO * 2)) ||
+      (rc = A(&g->dZ4T, B * NO * 2)) || (rc = A(&g->dZ, B * kHidden * 2)) || (rc = A(&g->dZT, B * kHidden * 2)) ||
       (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) || (rc = A(&g->count, 16)) ||
       (rc = A(&g->b_rays, B * 6 * 4)) || (rc = A(&g->b_labels, B * 4))) {
     sq_guide_destroy(g.release());
     return rc;
   }
   for (int l = 0; l < 3; ++l)
-    if ((rc = A(&g->H[l], B * kHidden * 2)) || (l < 2 && (rc = A(&g->HT[l], B * kHidden * 2)))) {
+    if ((rc = A(&g->H[l], B * kHidden * 2)) || (rc = A(&g->HT[l], B * kHidden * 2))) {
       sq_guide_destroy(g.release());
       return rc;
     }
