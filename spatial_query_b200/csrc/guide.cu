@@ -70,13 +70,7 @@ __global__ void features_kernel(const float* __restrict__ rays, uint32_t n, uint
   if (r >= B) return;
   float x[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (r < n) ray_features(rays + size_t(r) * 6, f, x);
-  __align__(16) bf16 v[8];
-#pragma unroll
-  for (uint32_t k = 0; k < 8; ++k) v[k] = __float2bfloat16_rn(k < 6 ? x[k] : 0.f);
-  uint4* row = reinterpret_cast<uint4*>(X + size_t(r) * kInPad);
-  row[0] = *reinterpret_cast<const uint4*>(v);
-#pragma unroll
-  for (uint32_t k = 1; k < kInPad / 8; ++k) row[k] = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t k = 0; k < kInPad; ++k) X[size_t(r) * kInPad + k] = __float2bfloat16_rn(k < 6 ? x[k] : 0.f);
   for (uint32_t k = 0; k < 6; ++k) XT[size_t(k) * B + r] = __float2bfloat16_rn(x[k]);
 }
 
@@ -633,11 +627,9 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uin
 int* g_err_slot(sq_ctx* ctx);
 
 // C[M x N] = A[M x K] * B[N x K]^T. a_rows / b_rows: allocated rows of A and B
-// (at least M and N; at least one box of 128 rows). into_zeros: C holds zeros,
-// so a product whose tiles leave SMs idle may be split along K, its shares
-// added in the L2.
+// (at least M and N; at least one box of 128 rows).
 int32_t gemm(sq_ctx* ctx, const bf16* A, uint64_t a_rows, uint32_t lda, const bf16* B, uint64_t b_rows, uint32_t ldb,
-             float* C, uint32_t M, uint32_t N, uint32_t K, uint32_t ldc, bool into_zeros = false) {
+             float* C, uint32_t M, uint32_t N, uint32_t K, uint32_t ldc) {
   if (M == 0 || N == 0) return SQ_OK;
   if (K == 0) {
     for (uint32_t r = 0; r < M; ++r) CK(cudaMemsetAsync(C + size_t(r) * ldc, 0, size_t(N) * 4, ctx->stream));
@@ -658,14 +650,8 @@ int32_t gemm(sq_ctx* ctx, const bf16* A, uint64_t a_rows, uint32_t lda, const bf
   int* err = g_err_slot(ctx);
   if (!err) return fail(ctx, SQ_ERR_CUDA, "error slot");
   dim3 grid((M + 127) / 128, (N + BN - 1) / BN);
-  // Shares of at least four K panels (one pipeline's depth), as many as fill
-  // the SMs once. A weight gradient of a hidden layer is one tile with K = the
-  // batch: 128 panels on one SM, 60 us per 8,192 rows; 32 shares take 7 us.
-  const uint32_t panels = (K + 63) / 64, tiles = grid.x * grid.y;
-  const bool split = into_zeros && tiles < uint32_t(ctx->sm_count) && panels >= 8;
-  if (split) grid.z = std::min<uint32_t>(panels / 4, std::max<uint32_t>(uint32_t(ctx->sm_count) / tiles, 1));
-  guide::gemm_tn_kernel<BN><<<grid, guide::kGemmThreads, smem, ctx->stream>>>(
-      ta, tb, C, int(M), int(N), int(K), int(ldc), split ? guide::kEpiReduce : guide::kEpiStore, err);
+  guide::gemm_tn_kernel<BN><<<grid, guide::kGemmThreads, smem, ctx->stream>>>(ta, tb, C, int(M), int(N), int(K),
+                                                                                int(ldc), guide::kEpiStore, err);
   ctx->launches++;
   CK(cudaGetLastError());
   return SQ_OK;
@@ -911,10 +897,8 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   transpose_colsum_kernel<<<dim3(B / 32, NO / 32), tb, 0, ctx->stream>>>(g->dZ4, g->dZ4T, g->G + g->ob4, B, NO);
   ctx->launches += 2;
   // backward
-  if ((rc = gemm(ctx, g->dZ4T, NO, B, g->HT[2], kHidden, B, g->G + g->oW4, NO, kHidden, B, kHidden, true)))
-    return rc;
-  CK(cudaMemsetAsync(g->dH, 0, size_t(B) * kHidden * 4, ctx->stream));
-  if ((rc = gemm(ctx, g->dZ4, B, NO, g->W4bT, kHidden, NO, g->dH, B, kHidden, NO, kHidden, true))) return rc;
+  if ((rc = gemm(ctx, g->dZ4T, NO, B, g->HT[2], kHidden, B, g->G + g->oW4, NO, kHidden, B, kHidden))) return rc;
+  if ((rc = gemm(ctx, g->dZ4, B, NO, g->W4bT, kHidden, NO, g->dH, B, kHidden, NO, kHidden))) return rc;
   const bf16* WT[3] = {nullptr, g->W2bT, g->W3bT};
   const size_t oW[3] = {g->oW1, g->oW2, g->oW3};
   for (int l = 2; l >= 0; --l) {
@@ -923,8 +907,7 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
     // dW_l = dZ^T [128 x B] * (input of layer l)^T [K x B]^T
     const bf16* inT = l == 0 ? g->XT : g->HT[l - 1];
     const uint32_t K_l = l == 0 ? kInPad : kHidden;
-    if ((rc = gemm(ctx, g->dZT, kHidden, B, inT, kHidden, B, g->G + oW[l], kHidden, K_l, B, K_l, true)))
-      return rc;
+    if ((rc = gemm(ctx, g->dZT, kHidden, B, inT, kHidden, B, g->G + oW[l], kHidden, K_l, B, K_l))) return rc;
     if (l > 0) {
       if ((rc = gemm(ctx, g->dZ, B, kHidden, WT[l], kHidden, kHidden, g->dH, B, kHidden, kHidden, kHidden))) return rc;
     }

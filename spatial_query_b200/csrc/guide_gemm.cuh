@@ -5,7 +5,7 @@
 // instruction) into a TMEM accumulator, and written back by four epilogue
 // warps through tcgen05.ld.
 //
-// One CTA per 128 x BN output tile and share of K; a 4-stage TMA -> MMA pipeline over K in
+// One CTA per 128 x BN output tile; a 4-stage TMA -> MMA pipeline over K in
 // 64-element panels: warp 0 lane 0 issues the loads, warp 1 lane 0 issues the
 // MMAs and frees each stage with tcgen05.commit, all four warps drain TMEM.
 // Rows and columns past M, N and K are zero-filled by TMA and masked at the
@@ -27,13 +27,8 @@ template <int BN> struct GemmSmem {
   static constexpr int bytes = kGemmStages * stage + 1024 /* barriers */ + 1024 /* alignment slack */;
 };
 
-// Epilogue modes: plain store, or add into C with reductions in the L2 (for
-// products split along K: the splits' CTAs add into a C zeroed before).
-enum GemmEpi : int { kEpiStore = 0, kEpiReduce = 1 };
-
-__device__ __forceinline__ void red_add4(float* dst, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
+// Epilogue modes: plain store, or add into C.
+enum GemmEpi : int { kEpiStore = 0, kEpiAccumulate = 1 };
 
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -52,10 +47,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * 128, n0 = blockIdx.y * BN;
-  // This CTA's share of the K panels: blockIdx.z of gridDim.z.
-  const int kt_all = (K + 63) / 64, kt_per = (kt_all + int(gridDim.z) - 1) / int(gridDim.z);
-  const int kt_0 = int(blockIdx.z) * kt_per, kt_n = min(kt_all - kt_0, kt_per);
-  if (kt_n <= 0 && gridDim.z > 1) return;  // the last splits of an uneven share
+  const int kt_n = (K + 63) / 64;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGemmStages; ++s) {
@@ -85,8 +77,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (*(volatile int*)s_err) break;
       uint8_t* sa = base + s * S::stage;
       umma::mbar_arrive_expect_tx(&full[s], S::stage);
-      umma::tma_load_2d(sa, &ta, &full[s], (kt_0 + kt) * 64, m0);
-      umma::tma_load_2d(sa + S::a_bytes, &tb, &full[s], (kt_0 + kt) * 64, n0);
+      umma::tma_load_2d(sa, &ta, &full[s], kt * 64, m0);
+      umma::tma_load_2d(sa + S::a_bytes, &tb, &full[s], kt * 64, n0);
     }
     *s_issued = kt;
   } else if (warp == 1 && lane == 0) {
@@ -123,15 +115,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (row < M) {
         float* dst = C + size_t(row) * ldc + n0 + c;
         const int lim = N - (n0 + c);
-        if (epi == kEpiReduce) {
-          if (lim >= 32 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+        if (epi == kEpiAccumulate) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) red_add4(dst + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < lim) atomicAdd(dst + j, v[j]);
-          }
+          for (int j = 0; j < 32; ++j)
+            if (j < lim) dst[j] += v[j];
         } else if (lim >= 32 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
