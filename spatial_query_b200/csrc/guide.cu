@@ -743,6 +743,8 @@ struct sq_guide {
   // shuffled training: permutation of the epoch and the gathered batch
   uint32_t* d_perm = nullptr;
   uint32_t perm_cap = 0;
+  float* loss_log = nullptr;  // an epoch's (loss, count) pairs, one per step
+  uint32_t log_cap = 0;
   float* b_rays = nullptr;
   int32_t* b_labels = nullptr;
 };
@@ -871,8 +873,7 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   const uint32_t B = g->B, NO = g->n_out;
   int32_t rc;
   CK(cudaMemsetAsync(g->G, 0, g->n_p * 4, ctx->stream));
-  CK(cudaMemsetAsync(g->loss, 0, 4, ctx->stream));
-  CK(cudaMemsetAsync(g->count, 0, 4, ctx->stream));
+  CK(cudaMemsetAsync(g->loss, 0, 8, ctx->stream));  // and count
   features_kernel<<<blocks_for(B, 256), 256, 0, ctx->stream>>>(d_rays, B, B, g->feat, g->X, g->XT);
   count_labels_kernel<<<std::min<uint32_t>(blocks_for(B, 256), 64), 256, 0, ctx->stream>>>(d_labels, B, g->n_buckets,
                                                                                             g->count);
@@ -916,14 +917,19 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
   return SQ_OK;
 }
 
+// The mean loss of a (loss sum, labelled rows) pair.
+float mean_loss(const float* pair) {
+  uint32_t c;
+  std::memcpy(&c, pair + 1, 4);
+  return c ? pair[0] / float(c) : 0.f;
+}
+
 int32_t read_loss(sq_guide* g, float* loss) {
   sq_ctx* ctx = g->ctx;
-  float s = 0.f;
-  uint32_t c = 0;
-  CK(cudaMemcpyAsync(&s, g->loss, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(&c, g->count, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  float pair[2];
+  CK(cudaMemcpyAsync(pair, g->loss, 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  *loss = c ? s / float(c) : 0.f;
+  *loss = mean_loss(pair);
   return SQ_OK;
 }
 
@@ -1004,6 +1010,7 @@ extern "C" int32_t sq_guide_destroy(sq_guide* g) {
   for (void* p : g->allocs) cudaFree(p);  // cudaFree waits for work using the memory
   if (g->d_leaf) cudaFree(g->d_leaf);
   if (g->d_perm) cudaFree(g->d_perm);
+  if (g->loss_log) cudaFree(g->loss_log);
   delete g;
   return SQ_OK;
 }
@@ -1067,11 +1074,12 @@ extern "C" int32_t sq_guide_create(sq_ctx* ctx, const sq_bvh* b, const sq_guide_
       (rc = A(&g->X, B * kInPad * 2)) || (rc = A(&g->XT, size_t(kHidden) * B * 2)) ||
       (rc = A(&g->Z, B * std::max<size_t>(NO, kHidden) * 4)) || (rc = A(&g->dZ4, B * NO * 2)) ||
       (rc = A(&g->dZ4T, B * NO * 2)) || (rc = A(&g->dZ, B * kHidden * 2)) || (rc = A(&g->dZT, B * kHidden * 2)) ||
-      (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) || (rc = A(&g->count, 16)) ||
+      (rc = A(&g->dH, B * kHidden * 4)) || (rc = A(&g->loss, 16)) ||
       (rc = A(&g->b_rays, B * 6 * 4)) || (rc = A(&g->b_labels, B * 4))) {
     sq_guide_destroy(g.release());
     return rc;
   }
+  g->count = reinterpret_cast<uint32_t*>(g->loss + 1);
   for (int l = 0; l < 3; ++l)
     if ((rc = A(&g->H[l], B * kHidden * 2)) || (rc = A(&g->HT[l], B * kHidden * 2))) {
       sq_guide_destroy(g.release());
@@ -1225,7 +1233,16 @@ extern "C" int32_t sq_guide_train_d(sq_guide* g, const float* d_rays, const int3
     CK(cudaMalloc(&g->d_perm, size_t(n) * 4));
     g->perm_cap = n;
   }
+  if (loss_per_epoch && g->log_cap < steps) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (g->loss_log) CK(cudaFree(g->loss_log));
+    g->loss_log = nullptr;
+    g->log_cap = 0;
+    CK(cudaMalloc(&g->loss_log, size_t(steps) * 8));
+    g->log_cap = steps;
+  }
   std::vector<uint32_t> perm(n);
+  std::vector<float> log(size_t(steps) * 2);
   for (uint32_t e = 0; e < epochs; ++e) {
     // A fresh shuffle per epoch (Fisher-Yates on SplitMix64, seeded by the
     // config seed and the optimiser step), so batches mix both ray kinds.
@@ -1242,12 +1259,17 @@ extern "C" int32_t sq_guide_train_d(sq_guide* g, const float* d_rays, const int3
                                                                           g->B, g->b_rays, g->b_labels);
       ctx->launches++;
       if ((rc = forward_backward(g, g->b_rays, g->b_labels))) return rc;
-      if (loss_per_epoch) {
-        float l = 0.f;
-        if ((rc = read_loss(g, &l))) return rc;
-        sum += l;
-      }
+      // Each step's loss stays on the device until the epoch's end: waiting
+      // for it here left the GPU idle between steps (11.2 -> 10.7 ms per 16
+      // steps of 8,192).
+      if (loss_per_epoch)
+        CK(cudaMemcpyAsync(g->loss_log + size_t(s) * 2, g->loss, 8, cudaMemcpyDeviceToDevice, ctx->stream));
       if ((rc = adam_step(g))) return rc;
+    }
+    if (loss_per_epoch && steps) {
+      CK(cudaMemcpyAsync(log.data(), g->loss_log, size_t(steps) * 8, cudaMemcpyDeviceToHost, ctx->stream));
+      CK(cudaStreamSynchronize(ctx->stream));
+      for (uint32_t s = 0; s < steps; ++s) sum += mean_loss(log.data() + size_t(s) * 2);
     }
     if (loss_per_epoch) loss_per_epoch[e] = steps ? float(sum / steps) : 0.f;
   }
