@@ -105,7 +105,13 @@ __global__ void count_labels_kernel(const int32_t* __restrict__ labels, uint32_t
 }
 
 // One row of logits per block: softmax cross-entropy against the label
-// (-1: ignored), dZ = (softmax - onehot) / n_labelled as bf16.
+// (-1: ignored), dZ = (softmax - onehot) / n_labelled as bf16. A thread holds
+// its columns (every 256th, at most 16 of at most 4,096) in registers, so each
+// logit is read and exponentiated once (read three times and exponentiated
+// twice from memory: 10.7 -> 9.9 ms per 16 steps of 8,192 x 4,096). The order of the sum of exponentials is
+// fixed: rounding dZ to bf16 and AdamW's first steps turn a sum in another order
+// into visibly different weights within a dozen steps.
+constexpr uint32_t kCeThreads = 256, kCeColumns = 4096 / kCeThreads;
 __global__ void softmax_ce_kernel(const float* __restrict__ Z, const float* __restrict__ b,
                                   const int32_t* __restrict__ labels, uint32_t n_out, uint32_t n_buckets,
                                   const uint32_t* count, bf16* dZ, float* loss_sum) {
@@ -120,7 +126,13 @@ __global__ void softmax_ce_kernel(const float* __restrict__ Z, const float* __re
     return;
   }
   float m = -INFINITY;
-  for (uint32_t j = threadIdx.x; j < n_buckets; j += blockDim.x) m = fmaxf(m, z[j] + b[j]);
+  float v[kCeColumns];
+#pragma unroll
+  for (uint32_t k = 0; k < kCeColumns; ++k) {
+    const uint32_t j = threadIdx.x + k * kCeThreads;
+    v[k] = j < n_buckets ? z[j] + b[j] : -INFINITY;
+    m = fmaxf(m, v[k]);
+  }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) red[warp] = m;
   __syncthreads();
@@ -128,7 +140,9 @@ __global__ void softmax_ce_kernel(const float* __restrict__ Z, const float* __re
   for (int w = 1; w < nw; ++w) m = fmaxf(m, red[w]);
   __syncthreads();
   float s = 0.f;
-  for (uint32_t j = threadIdx.x; j < n_buckets; j += blockDim.x) s += expf(z[j] + b[j] - m);
+#pragma unroll
+  for (uint32_t k = 0; k < kCeColumns; ++k)
+    if (threadIdx.x + k * kCeThreads < n_buckets) s += v[k] = expf(v[k] - m);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) red[warp] = s;
   __syncthreads();
@@ -136,9 +150,12 @@ __global__ void softmax_ce_kernel(const float* __restrict__ Z, const float* __re
   for (int w = 0; w < nw; ++w) s += red[w];
   const float inv_n = 1.0f / float(max(*count, 1u));
   const float inv_s = 1.0f / s;
-  for (uint32_t j = threadIdx.x; j < n_out; j += blockDim.x) {
+#pragma unroll
+  for (uint32_t k = 0; k < kCeColumns; ++k) {
+    const uint32_t j = threadIdx.x + k * kCeThreads;
+    if (j >= n_out) break;
     float g = 0.f;
-    if (j < n_buckets) g = expf(z[j] + b[j] - m) * inv_s - (j == uint32_t(y) ? 1.f : 0.f);
+    if (j < n_buckets) g = v[k] * inv_s - (j == uint32_t(y) ? 1.f : 0.f);
     dz[j] = __float2bfloat16_rn(g * inv_n);
   }
   if (threadIdx.x == 0) atomicAdd(loss_sum, logf(s) + m - (z[y] + b[y]));
@@ -893,7 +910,7 @@ int32_t forward_backward(sq_guide* g, const float* d_rays, const int32_t* d_labe
     in_k = kHidden;
   }
   if ((rc = gemm(ctx, g->H[2], B, kHidden, g->W4b, NO, kHidden, g->Z, B, NO, kHidden, NO))) return rc;
-  softmax_ce_kernel<<<B, 256, 0, ctx->stream>>>(g->Z, g->P + g->ob4, d_labels, NO, g->n_buckets, g->count, g->dZ4,
+  softmax_ce_kernel<<<B, kCeThreads, 0, ctx->stream>>>(g->Z, g->P + g->ob4, d_labels, NO, g->n_buckets, g->count, g->dZ4,
                                                 g->loss);
   transpose_colsum_kernel<<<dim3(B / 32, NO / 32), tb, 0, ctx->stream>>>(g->dZ4, g->dZ4T, g->G + g->ob4, B, NO);
   ctx->launches += 2;
