@@ -5,7 +5,7 @@
 // instruction) into a TMEM accumulator, and written back by four epilogue
 // warps through tcgen05.ld.
 //
-// One CTA per 128 x BN output tile; a 4-stage TMA -> MMA pipeline over K in
+// One CTA per 128 x BN output tile; a TMA -> MMA pipeline over K in
 // 64-element panels: warp 0 lane 0 issues the loads, warp 1 lane 0 issues the
 // MMAs and frees each stage with tcgen05.commit, all four warps drain TMEM.
 // Rows and columns past M, N and K are zero-filled by TMA and masked at the
@@ -17,10 +17,9 @@
 namespace sq {
 namespace guide {
 
-constexpr int kGemmStages = 4;
 constexpr int kGemmThreads = 128;
 
-template <int BN> struct GemmSmem {
+template <int BN, int kGemmStages> struct GemmSmem {
   static constexpr int a_bytes = 128 * 128;  // 128 rows x 64 bf16
   static constexpr int b_bytes = BN * 128;
   static constexpr int stage = a_bytes + b_bytes;
@@ -30,11 +29,11 @@ template <int BN> struct GemmSmem {
 // Epilogue modes: plain store, or add into C.
 enum GemmEpi : int { kEpiStore = 0, kEpiAccumulate = 1 };
 
-template <int BN>
+template <int BN, int kGemmStages>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_tn_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float* __restrict__ C,
                    int M, int N, int K, int ldc, int epi, int* err) {
-  using S = GemmSmem<BN>;
+  using S = GemmSmem<BN, kGemmStages>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = umma::smem_u32(smem_raw);
   uint8_t* base = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
