@@ -64,13 +64,14 @@ constexpr int kThreads = 128;
 // instantiation, SQ_LAYOUT_BINARY_REGTOP, which the autotuner can pick):
 //  * SQ_POSTPONE_LEAVES: a lane that reaches a leaf holds it and keeps
 //    descending until the whole warp holds leaves (Aila and Laine's
-//    speculative traversal): 0.697 ms against 0.621 ms per 1,048,576 rays;
-//    the nodes it visits before the leaf's hit tightens the limit cost more
-//    than the leaf tests gain from running together.
+//    speculative traversal): the nodes it visits before the leaf's hit
+//    tightens the limit cost more than the leaf tests gain from running
+//    together.
 //  * SQ_REG_TOP (with postponed leaves): the stack's top entry in registers,
-//    older entries in the shared-memory stack: 0.729 ms; five more registers
-//    per thread cut the resident blocks from nine to eight, and the saved
-//    shared-memory round trip is short next to a node fetch from L2.
+//    older entries in the shared-memory stack: 0.672-0.682 ms per 1,048,576
+//    rays against 0.436 ms for the warp-stepped walk; the saved shared-memory
+//    round trip is short next to a node fetch from L2, and these walks have no
+//    helping lanes.
 #ifndef SQ_POSTPONE_LEAVES
 #define SQ_POSTPONE_LEAVES 0
 #endif
@@ -83,7 +84,7 @@ constexpr int kThreads = 128;
 // on a node stay on the same path; 0 (the default): each lane's own nearer
 // child first (WALK = 2 builds it as SQ_LAYOUT_BINARY_VOTE). Measured on the
 // terrain's 1,048,576 rays (answers identical):
-// 0.652 ms against 0.616 ms for each lane's own order; the vote costs every
+// 0.490 ms against 0.436 ms for each lane's own order; the vote costs every
 // node step, and a lane outvoted takes its farther child first.
 #ifndef SQ_WARP_ORDER
 #define SQ_WARP_ORDER 0
@@ -92,10 +93,10 @@ constexpr int kThreads = 128;
 // triangles and rays, each pair by the other values alike): answers written
 // and queries loaded once 1 / 4 / 8 / 16 / 24 lanes are free 705 / 641 / 625
 // / 615 / 617 us; a leaf pass once 1/2, 2/3, 1/3 or 1/4 of the walking lanes
-// wait at one 615 / 627 / 625 / 633 us.
+// wait at one 615 / 627 / 625 / 633 us (before the free lanes helped).
 constexpr int kRefill = 16;     // free lanes (of 32) before the warp refills them
 constexpr int kLeafWeight = 2;  // a leaf pass when waiting lanes x this reach the walking lanes
-constexpr int kMaxStack = 96;  // deepest tree accepted (96 KB of stack per block)
+constexpr int kMaxStack = 96;  // deepest tree accepted (96 KB of stack per block, 144 KB for f64 scenes)
 
 // 16-byte vectors of a record of `words` words: records longer than one
 // vector are padded to whole 32-byte sectors, so that each is read with
